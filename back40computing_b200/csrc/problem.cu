@@ -16,6 +16,12 @@ namespace rt {
 int alloc_dev(void **p, size_t bytes, const char *what)
 {
     cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        int device = -1;
+        if (cudaGetDevice(&device) == cudaSuccess) release_conversion_memory(device);
+        e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;

@@ -135,6 +135,8 @@ struct DeviceGuard {
 inline const int32_t *source_slot(const b40c_bfs_problem *p) { return p->h_src_ring + 2 * p->ring_pos; }
 
 int alloc_dev(void **p, size_t bytes, const char *what);
+// Returns the memory the device's COO conversions keep between calls (coo_to_csr.cu).
+void release_conversion_memory(int device);
 void free_vf(VertexFrontier &f);
 void free_ef(EdgeFrontier &f);
 int ensure_vf(b40c_bfs_problem *p, int i, int64_t cap);

@@ -46,6 +46,24 @@ def test_matches_stable_host_conversion(n, m):
     assert np.array_equal(ci, want_ci)
 
 
+# one, two and three digits of every width class; tiles of 2048 and 16384 edges
+# with full and ragged ends, the switch between them (148 SMs x 16384 edges); rows
+# all equal, all different mod 32, and uniform
+@pytest.mark.parametrize("n,m", [(31, 2047), (32, 2048), (33, 2049), (2048, 6143), (2049, 70001), (1 << 22, 4097),
+                                 ((1 << 22) + 1, 200003), (1000, 148 * 16384 - 1), (5000, 148 * 16384),
+                                 (1 << 21, 148 * 16384 + 1)])
+@pytest.mark.parametrize("kind", ["uniform", "one-row", "cyclic"])
+def test_radix_pass_edges(n, m, kind):
+    rng = np.random.default_rng(m)
+    rows = {"uniform": rng.integers(0, n, m), "one-row": np.full(m, n - 1), "cyclic": np.arange(m) % n}[kind]
+    cols = rng.integers(0, n, m)
+    rc, ro, ci = _device(n, rows, cols)
+    assert rc == 0
+    want_ro, want_ci = _host_csr(n, rows, cols)
+    assert np.array_equal(ro, want_ro)
+    assert np.array_equal(ci, want_ci)
+
+
 def test_rejects_ids_out_of_range():
     rows = np.array([0, 1, 5], np.int32)
     cols = np.array([1, 2, 0], np.int32)
