@@ -38,10 +38,9 @@ namespace dev {
 
 constexpr int kChunkMax = 2048;   // edges (or edge-frontier items) per sub-round
 constexpr int kChunkGrain = 256;  // CTA ranges start at multiples of this; granularity of the cf index
-// With a sub-grid threshold (p.subgrid_edges), mid-size top-down levels (more
-// edges than a solo level, at most the threshold) of a persistent search run on
-// the first kSubgridCtas CTAs, which synchronise among themselves; the rest of
-// the grid waits at the grid barrier.
+// With a sub-grid threshold (p.team_edges > 0), the mid-size top-down levels
+// that a team of CTAs runs (team_phase) have at most that many edges and take at
+// most this many CTAs.
 constexpr int kSubgridCtas = 16;
 
 // emit_frontier: output entries whose degree spans more chunks than this have
@@ -50,11 +49,12 @@ constexpr unsigned kCfSerialChunks = 8;
 
 template <int B, bool PRED>
 struct ExpandSmem {
+    static constexpr int kEntries = kChunkMax;
     // per-sub-round run tables; after the gather they hold the sub-round's
     // output (colstart = row start, rel = degree of each discovered vertex)
-    int32_t colstart[kChunkMax + 2];
-    int32_t rel[kChunkMax + 2];
-    int32_t vert[PRED ? kChunkMax + 2 : 1];
+    int32_t colstart[kEntries + 2];
+    int32_t rel[kEntries + 2];
+    int32_t vert[PRED ? kEntries + 2 : 1];
     alignas(16) uint16_t own[kChunkMax];  // position -> run j owning it
     int32_t out[kChunkMax];   // discovered vertices of the sub-round
     alignas(16) int32_t stage[kChunkMax + 16];  // bulk-staged run (sub-round inside one list)
@@ -62,6 +62,9 @@ struct ExpandSmem {
     int32_t out_count;
     int32_t flag;             // a vertex was labelled by this CTA in the current pass
     int32_t q, E;
+    uint32_t error;                    // the error word and
+    int32_t depth_limit;               // depth limit as read at the start of the pass
+    unsigned long long team_sum;       // a team barrier's sums
     unsigned long long visited_edges;  // degree sum of the vertices visited up to this pass
     int32_t prev_bu;                   // the previous level ran bottom-up
     uint32_t *mask;                    // the visited-mask buffer of this pass (mask or mask_alt)
@@ -212,16 +215,20 @@ __device__ __forceinline__ unsigned long long cta_exclusive_scan(unsigned long l
     }
     if (lane == 31) warp_buf[warp] = incl;
     __syncthreads();
-    unsigned long long wpre = 0, tot = 0;
+    // every warp scans the warps' sums with its own lanes: one shared load each,
+    // where a loop over them costs B / 32 loads by B / 32 warps
+    constexpr int NW = B / 32;
+    const unsigned long long own = lane < NW ? warp_buf[lane] : 0ull;
+    unsigned long long pre = own;
 #pragma unroll
-    for (int w = 0; w < B / 32; w++) {
-        unsigned long long t = warp_buf[w];
-        if (w < warp) wpre += t;
-        tot += t;
+    for (int off = 1; off < NW; off <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, pre, off);
+        if (lane >= off) pre += y;
     }
+    *total = __shfl_sync(0xffffffffu, pre, NW - 1);
+    const unsigned long long before = __shfl_sync(0xffffffffu, pre - own, warp);
     __syncthreads();
-    *total = tot;
-    return wpre + incl - x;
+    return before + incl - x;
 }
 
 // Optional warp culling: among lanes holding the same vertex only the lowest stays valid.
@@ -232,9 +239,14 @@ __device__ __forceinline__ bool warp_cull(bool valid, int v)
     return valid && (__ffs(peers) - 1 == lane);
 }
 
+// Passes of fewer items than this test without the pre-check: they have few
+// duplicates, and its round trip costs more than the atomics it saves.
+constexpr int kPrecheckItems = 1 << 16;
+
 // Discovery of up to U gathered neighbours per thread, in overlapped phases
-// (visited-word pre-checks, then atomic test-and-sets, then the CSR rows of
-// the winners) so each thread keeps all of its memory operations in flight.
+// (visited-word pre-checks, then atomic test-and-sets beside the CSR rows) so
+// each thread keeps all of its memory operations in flight.  `items`: the
+// pass's positions (kPrecheckItems).
 // A winner is labelled and, when it has edges, appended to the sub-round's
 // output (s.out = vertex, s.colstart = row start, s.rel = degree; the run
 // tables are consumed by then).  With LEAVES (vertex-frontier searches) the
@@ -245,11 +257,11 @@ __device__ __forceinline__ bool warp_cull(bool valid, int v)
 template <int B, bool PRED, int U, bool LISTS = false, bool LEAVES = false>
 __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B, PRED> &s, const int (&v)[U],
                                                const int (&u)[U], const bool (&valid)[U], const bool (&active)[U],
-                                               int label_value, bool precheck = true)
+                                               int label_value, int items)
 {
     bool go[U];
     unsigned word[U];
-    precheck = precheck && p.precheck && !(LISTS && s.ul_in >= 0);
+    const bool precheck = p.precheck && items >= kPrecheckItems && !(LISTS && s.ul_in >= 0);
     uint32_t *hist = s.hist;
 #pragma unroll
     for (int t = 0; t < U; t++) {
@@ -266,32 +278,45 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
         if (go[t] && precheck) word[t] = p.precheck == 2 ? ld_cg(s.mask + (v[t] >> 5)) : ld_mask(s.mask + (v[t] >> 5));
     }
     bool found[U];
+    int r0[U], r1[U];
     if (LISTS && s.ul_in >= 0) {
         // after a bottom-up list-mode level the visited mask is not kept: the
         // labels decide (a distance search's unreached vertices hold -1)
 #pragma unroll
         for (int t = 0; t < U; t++) {
             found[t] = false;
+            r0[t] = r1[t] = 0;
             if (go[t] && ld_cg(p.labels + v[t]) == -1) found[t] = atomicCAS(p.labels + v[t], -1, label_value) == -1;
+            if (found[t]) {
+                r0[t] = ld_ro(p.row_offsets + v[t]);
+                r1[t] = ld_ro(p.row_offsets + v[t] + 1);
+            }
         }
     } else {
+        // the rows are loaded beside the test-and-set, for losers too: a level
+        // of this size waits for round trips, not for their bandwidth
+        unsigned old[U];
 #pragma unroll
         for (int t = 0; t < U; t++) {
             const unsigned bit = 1u << (v[t] & 31);
-            found[t] = false;
-            if (go[t] && !(word[t] & bit)) found[t] = !(atomicOr(s.mask + (v[t] >> 5), bit) & bit);
+            go[t] = go[t] && !(word[t] & bit);
+            old[t] = ~0u;
+            if (go[t]) old[t] = atomicOr(s.mask + (v[t] >> 5), bit);
         }
-    }
-    int r0[U], r1[U];
 #pragma unroll
-    for (int t = 0; t < U; t++) {
-        r0[t] = r1[t] = 0;
-        if (found[t]) {
-            p.labels[v[t]] = PRED ? u[t] : label_value;
-            r0[t] = ld_ro(p.row_offsets + v[t]);
-            r1[t] = ld_ro(p.row_offsets + v[t] + 1);
+        for (int t = 0; t < U; t++) {
+            r0[t] = r1[t] = 0;
+            if (go[t]) {
+                r0[t] = ld_ro(p.row_offsets + v[t]);
+                r1[t] = ld_ro(p.row_offsets + v[t] + 1);
+            }
         }
+#pragma unroll
+        for (int t = 0; t < U; t++) found[t] = !((old[t] >> (v[t] & 31)) & 1u);
     }
+#pragma unroll
+    for (int t = 0; t < U; t++)
+        if (found[t]) p.labels[v[t]] = PRED ? u[t] : label_value;
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int t = 0; t < U; t++) {
@@ -329,15 +354,16 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
 // A tile whose output ends past `skip_above` edges of the pass total only
 // counts: the caller passes the edge total beyond which the next level is
 // certain to run bottom-up (which never reads the frontier).  All threads must
-// call it.
-template <int B, typename Smem>
+// call it.  With WRITE_V = false the entries' vertices are not written (distance
+// searches never read them).
+template <int B, bool WRITE_V = true, typename Smem>
 __device__ __forceinline__ void emit_frontier(const BfsParams &p, Smem &s, int pass, const VertexFrontier &vout,
                                               unsigned long long *qe_out, bool lookback = true,
                                               unsigned long long skip_above = ~0ull)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cnt = s.out_count;
-    constexpr int PER = kChunkMax / B;
+    constexpr int PER = Smem::kEntries / B;
     const int per = (cnt + B - 1) / B;
     const int jb = min(tid * per, cnt), je = min(jb + per, cnt);
     unsigned my_deg = 0;
@@ -386,7 +412,7 @@ __device__ __forceinline__ void emit_frontier(const BfsParams &p, Smem &s, int p
     for (int j = jb; j < je; j++) {
         const unsigned deg = (unsigned)s.rel[j];
         if ((int)g < p.vcap) {
-            vout.v[g] = s.out[j];
+            if (WRITE_V) vout.v[g] = s.out[j];
             vout.col[g] = s.colstart[j];
             vout.P[g] = (int)d;
             // cf[c] = g for the chunks c starting inside [d, d + deg); long runs
@@ -457,6 +483,31 @@ __device__ __forceinline__ void cta_range(int n, int part, int parts, int &rs, i
     re = (b == G - 1) ? n : (int)((long long)n * (b + 1) / G / kChunkGrain * kChunkGrain);
 }
 
+// The run tables' position -> entry map (s.own) from the entries' first
+// positions s.rel[0..n], s.rel[n] the end: short lists by their lane, long ones
+// by the whole warp (against a binary search per thread: 0.7 -> 0.3 us of a
+// level of short lists).  All threads call it; the caller's barriers publish rel
+// before and own after.
+template <int B, typename Smem>
+__device__ __forceinline__ void fill_owners(Smem &s, int n)
+{
+    const int lane = threadIdx.x & 31;
+    for (int jb = threadIdx.x & ~31; jb < n; jb += B) {
+        const int j = jb + lane;
+        const int lo = j < n ? s.rel[j] : 0, hi = j < n ? s.rel[j + 1] : 0;
+        const bool is_long = hi - lo > 16;
+        if (!is_long)
+            for (int x = lo; x < hi; x++) s.own[x] = (uint16_t)j;
+        unsigned todo = __ballot_sync(0xffffffffu, is_long);
+        while (todo) {
+            const int L = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int a = __shfl_sync(0xffffffffu, lo, L), b = __shfl_sync(0xffffffffu, hi, L);
+            for (int x = a + lane; x < b; x += 32) s.own[x] = (uint16_t)(jb + L);
+        }
+    }
+}
+
 // ------------------------------------------------------------------------------------
 // Edge-balanced expansion of the CTA's range of a vertex frontier's flattened
 // edge space, in sub-rounds of kChunkMax positions.
@@ -470,7 +521,7 @@ template <int B, bool PRED, bool FUSED_CULL, bool LISTS = false>
 __device__ __forceinline__ void expand_range(const BfsParams &p, const VertexFrontier &in, ExpandSmem<B, PRED> &s,
                                              int level, int pass, const VertexFrontier &vout,
                                              const EdgeFrontier &eout, unsigned long long *qe_out,
-                                             unsigned &bar_phase, int part, int parts, bool defer_emit = false,
+                                             unsigned &bar_phase, int part, int parts,
                                              unsigned long long skip_above = ~0ull)
 {
     const int tid = threadIdx.x;
@@ -481,8 +532,7 @@ __device__ __forceinline__ void expand_range(const BfsParams &p, const VertexFro
     if (rs >= re) return;
     int i_cur = ld_cg(in.cf + rs / kChunkGrain);  // entry owning position rs
     if (FUSED_CULL) stamp(p, pass, 0);
-    // sub-round length: policy.chunk_edges (a solo level kept in shared memory is one full sub-round)
-    const int chunk = defer_emit ? kChunkMax : min(max(p.chunk_edges, 256), kChunkMax);
+    const int chunk = min(max(p.chunk_edges, 256), kChunkMax);  // sub-round length
     for (int cs = rs; cs < re; cs += chunk) {
         const int ce = min(cs + chunk, re);
         const int len = ce - cs;
@@ -571,30 +621,8 @@ __device__ __forceinline__ void expand_range(const BfsParams &p, const VertexFro
                 }
             }
         } else {
-            // ---- owner map: thread t resolves positions [t*PER, t*PER + PER)
-            // (binary search for the first, then a walk over run starts) -----------
-            __syncthreads();
-            const int x0 = tid * PER;
-            if (x0 < len) {
-                int lo = 0, hi = k - 1;  // last j with rel[j] <= x0
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s.rel[mid] <= x0) lo = mid; else hi = mid - 1;
-                }
-                int j = lo;
-                int next = s.rel[j + 1];
-#pragma unroll
-                for (int t = 0; t < PER; t++) {
-                    const int x = x0 + t;
-                    if (x < len) {
-                        while (x >= next) {
-                            j++;
-                            next = s.rel[j + 1];
-                        }
-                        s.own[x] = (uint16_t)j;
-                    }
-                }
-            }
+            __syncthreads();  // rel[k] is written
+            fill_owners<B>(s, k);
         }
         if (!__syncthreads_and(staged)) {
             // the copy did not land in time: report it, give the copy still in
@@ -643,71 +671,13 @@ __device__ __forceinline__ void expand_range(const BfsParams &p, const VertexFro
         }
         __syncthreads();  // run tables consumed: they now collect the sub-round's output
         if (first) stamp(p, pass, 3);
-        discover_batch<B, PRED, PER, LISTS, true>(p, s, v, u, valid, active, level + 1);
+        discover_batch<B, PRED, PER, LISTS, true>(p, s, v, u, valid, active, level + 1, E);
         __syncthreads();
         if (first) stamp(p, pass, 4);
-        if (defer_emit) return;  // single sub-round (the caller checked): the output stays in s.out / colstart / rel
         emit_frontier<B>(p, s, pass, vout, qe_out, true, skip_above);
         __syncthreads();
         if (first) stamp(p, pass, 5);
     }
-}
-
-// Solo levels (CTA 0 alone, one sub-round each) can pass their frontier from
-// one level to the next in shared memory.  A level's discoveries sit in
-// s.out / colstart / rel (n entries: vertex, row start, degree); the next
-// level turns them in place into its run tables (rel = degree prefix with
-// rel[n] = E, colstart = row start, vert = vertex) and runs from there, with
-// no frontier, counter or chunk-index traffic.  solo_level_smem runs such a
-// level: owner map, gather, discovery (atomic test-and-set without the
-// visited-word pre-check), output back in s.out / colstart / rel.
-template <int B, bool PRED, bool LISTS>
-__device__ __forceinline__ void solo_level_smem(const BfsParams &p, ExpandSmem<B, PRED> &s, int level, int n, int E)
-{
-    const int tid = threadIdx.x;
-    constexpr int PER = kChunkMax / B;
-    {
-        const int x0 = tid * PER;
-        if (x0 < E) {
-            int lo = 0, hi = n - 1;  // last j with rel[j] <= x0
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (s.rel[mid] <= x0) lo = mid; else hi = mid - 1;
-            }
-            int j = lo;
-            int next = s.rel[j + 1];
-#pragma unroll
-            for (int t = 0; t < PER; t++) {
-                const int x = x0 + t;
-                if (x < E) {
-                    while (x >= next) {
-                        j++;
-                        next = s.rel[j + 1];
-                    }
-                    s.own[x] = (uint16_t)j;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    int v[PER], u[PER];
-    bool valid[PER], active[PER];
-#pragma unroll
-    for (int t = 0; t < PER; t++) {
-        const int x = t * B + tid;
-        active[t] = t * B < E;
-        valid[t] = x < E;
-        v[t] = -1;
-        u[t] = -1;
-        if (valid[t]) {
-            const int j = s.own[x];
-            v[t] = ld_stream(p.column_indices + s.colstart[j] + (x - s.rel[j]));
-            if (PRED) u[t] = s.vert[j];
-        }
-    }
-    __syncthreads();  // run tables consumed: they now collect the level's output
-    discover_batch<B, PRED, PER, LISTS, true>(p, s, v, u, valid, active, level + 1, false);
-    __syncthreads();
 }
 
 // Contraction of the CTA's range of an edge frontier (q items), in sub-rounds
@@ -738,7 +708,7 @@ __device__ __forceinline__ void contract_range(const BfsParams &p, ExpandSmem<B,
             u[t] = (PRED && valid[t]) ? ld_cg(in.pred + i) : -1;
         }
         __syncthreads();
-        discover_batch<B, PRED, PER>(p, s, v, u, valid, active, level);
+        discover_batch<B, PRED, PER>(p, s, v, u, valid, active, level, q);
         __syncthreads();
         emit_frontier<B>(p, s, pass, p.vf[0], qe_out);
         __syncthreads();
@@ -846,18 +816,18 @@ __device__ __forceinline__ int warp_slice0(int warp) { return warp * (int)gridDi
 
 // Visited test of one warp's batch of PER neighbours per lane (pre-check
 // loads, atomic test-and-set, the CSR rows of the winners; each winner is
-// labelled), then the winners with edges appended to the warp's output
-// (bv / bc / bd, `count` entries of at most `cap`, flushed to the vertex
-// frontier first when the batch could overrun it).  With LEAVES the winners
-// without edges are added to total_queued (vertex-frontier strategies queue
-// every discovered vertex, expand_contract_atomic/cta.cuh:432-466).  Returns
-// whether this lane labelled a vertex.  All 32 lanes call it.
-template <int PER, bool PRED, bool LEAVES, int CAP>
+// labelled, with pred(t) in predecessor searches), then the winners with edges
+// appended to the warp's output (bv / bc / bd, `count` entries of at most
+// `cap`, flushed to the vertex frontier first when the batch could overrun it).
+// With LEAVES the winners without edges are added to total_queued
+// (vertex-frontier strategies queue every discovered vertex,
+// expand_contract_atomic/cta.cuh:432-466).  Returns whether this lane labelled a
+// vertex.  All 32 lanes call it.
+template <int PER, bool PRED, bool LEAVES, int CAP, typename PredOf>
 __device__ __forceinline__ bool warp_discover(const BfsParams &p, uint32_t *mask, const int (&v)[PER],
-                                             const int (&u)[PER], const bool (&go)[PER], int label_value,
-                                             int32_t *bv, int32_t *bc, int32_t *bd, int &count,
-                                             const VertexFrontier &vout, unsigned long long *qe_out,
-                                             unsigned long long skip_above = ~0ull)
+                                             const bool (&go)[PER], int label_value, PredOf pred, int32_t *bv,
+                                             int32_t *bc, int32_t *bd, int &count, const VertexFrontier &vout,
+                                             unsigned long long *qe_out, unsigned long long skip_above = ~0ull)
 {
     const int lane = threadIdx.x & 31;
     const int pre = p.precheck;
@@ -879,7 +849,7 @@ __device__ __forceinline__ bool warp_discover(const BfsParams &p, uint32_t *mask
     for (int t = 0; t < PER; t++) {
         r0[t] = deg[t] = 0;
         if (found[t]) {
-            p.labels[v[t]] = PRED ? u[t] : label_value;
+            p.labels[v[t]] = PRED ? pred(t) : label_value;
             r0[t] = ld_ro(p.row_offsets + v[t]);
             deg[t] = ld_ro(p.row_offsets + v[t] + 1);
             any = true;
@@ -936,8 +906,8 @@ __device__ __forceinline__ void contract_range_warp(const BfsParams &p, ExpandSm
                                                     const EdgeFrontier &in, int level, const VertexFrontier &vout,
                                                     unsigned long long *qe_out)
 {
-    // eight items per lane whatever the CTA size: with 512-thread CTAs a warp's
-    // output holds half a slice, and warp_discover appends the winners in halves
+    // eight items per lane whatever the CTA size: with larger CTAs a warp's
+    // output holds less than a slice, and warp_discover appends the winners in parts
     constexpr int PER = 8;
     constexpr int NW = B / 32;
     constexpr int S = 32 * PER;           // items per slice
@@ -952,16 +922,16 @@ __device__ __forceinline__ void contract_range_warp(const BfsParams &p, ExpandSm
     const long long stride = (long long)gridDim.x * NW * S;
     for (long long b64 = (long long)warp_slice0(warp) * S; b64 < re; b64 += stride) {
         const int base = (int)b64;
-        int v[PER], u[PER];
+        int v[PER];
         bool go[PER];
 #pragma unroll
         for (int t = 0; t < PER; t++) {
             const int i = base + t * 32 + lane;
             go[t] = i < re;
             v[t] = go[t] ? ld_cg(in.v + i) : -1;
-            u[t] = (PRED && go[t]) ? ld_cg(in.pred + i) : -1;
         }
-        any |= warp_discover<PER, PRED, false, CAP>(p, s.mask, v, u, go, level, bv, bc, bd, count, vout, qe_out);
+        const auto pred = [&](int t) { return ld_cg(in.pred + base + t * 32 + lane); };
+        any |= warp_discover<PER, PRED, false, CAP>(p, s.mask, v, go, level, pred, bv, bc, bd, count, vout, qe_out);
     }
     if (count) warp_emit(p, bv, bc, bd, count, vout, qe_out);
     if (__any_sync(0xffffffffu, any) && lane == 0) s.flag = 1;  // benign race: every writer stores 1
@@ -973,11 +943,11 @@ __device__ __forceinline__ void contract_range_warp(const BfsParams &p, ExpandSm
 // marking its first slice position in `own` (cleared first), which a warp
 // max-scan then fills: position r belongs to the largest mark at or before r
 // (the entries start in increasing order).  tcol[k] + r is the column index
-// of slice position r in entry k's list; tver[k] is entry k's vertex.  All
-// 32 lanes call it, after every lane has finished reading the tables.
-template <bool PRED>
-__device__ __forceinline__ void warp_slice_map(const VertexFrontier &in, int q, int x0, int len, uint16_t *own,
-                                               int32_t *tcol, int32_t *tver)
+// of slice position r in entry k's list; entry k is the frontier's entry
+// returned + k.  All 32 lanes call it, after every lane has finished reading
+// the tables.
+__device__ __forceinline__ int warp_slice_map(const VertexFrontier &in, int q, int x0, int len, uint16_t *own,
+                                              int32_t *tcol)
 {
     const int lane = threadIdx.x & 31;
     reinterpret_cast<uint4 *>(own)[lane] = make_uint4(0u, 0u, 0u, 0u);
@@ -987,11 +957,10 @@ __device__ __forceinline__ void warp_slice_map(const VertexFrontier &in, int q, 
     for (int i = i0;; i += 32) {
         const int j = i + lane;
         int Pj = INT_MAX;
-        int cj = 0, vj = -1;
+        int cj = 0;
         if (j < q) {
             Pj = ld_cg(in.P + j);
             cj = ld_cg(in.col + j);
-            if (PRED) vj = ld_cg(in.v + j);
         }
         const bool inside = Pj < x0 + len;  // the inside lanes form a prefix (P increases)
         const unsigned in_mask = __ballot_sync(0xffffffffu, inside);
@@ -1000,7 +969,6 @@ __device__ __forceinline__ void warp_slice_map(const VertexFrontier &in, int q, 
             const int start = max(Pj, x0) - x0;
             own[start] = (uint16_t)k;
             tcol[k] = cj + (max(Pj, x0) - Pj) - start;  // + slice position = column index
-            if (PRED) tver[k] = vj;
         }
         n += __popc(in_mask);
         if (in_mask != 0xffffffffu || i + 32 >= q) break;
@@ -1027,28 +995,22 @@ __device__ __forceinline__ void warp_slice_map(const VertexFrontier &in, int q, 
     w.w = e[6] | (e[7] << 16);
     reinterpret_cast<uint4 *>(own)[lane] = w;
     __syncwarp();
+    return i0;
 }
 
 // Lane positions (h * PB + t) * 32 + lane, t < PB, of a slice of `len`
-// positions: the gathered neighbour (a coalesced read along a run) and its
-// predecessor, from the warp's tables.
-template <int PB, bool PRED>
+// positions: the gathered neighbours (a coalesced read along a run), from the
+// warp's tables.
+template <int PB>
 __device__ __forceinline__ void warp_slice_gather(const BfsParams &p, int h, int len, const uint16_t *own,
-                                                  const int32_t *tcol, const int32_t *tver, int (&v)[PB],
-                                                  int (&u)[PB], bool (&go)[PB])
+                                                  const int32_t *tcol, int (&v)[PB], bool (&go)[PB])
 {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int t = 0; t < PB; t++) {
         const int r = (h * PB + t) * 32 + lane;
         go[t] = r < len;
-        v[t] = -1;
-        u[t] = -1;
-        if (go[t]) {
-            const int k = own[r];
-            v[t] = ld_stream(p.column_indices + tcol[k] + r);
-            if (PRED) u[t] = tver[k];
-        }
+        v[t] = go[t] ? ld_stream(p.column_indices + tcol[own[r]] + r) : -1;
     }
 }
 
@@ -1068,22 +1030,21 @@ __device__ __forceinline__ void warp_slice_gather(const BfsParams &p, int h, int
 // gathered neighbours (and their predecessors) are written to the edge
 // frontier `eout` at their flattened positions instead: the reference's
 // two-phase expansion (two_phase/expand_atomic/cta.cuh:215-423).
-// Predecessor searches with CTAs of more than 256 threads keep the CTA-wide
-// sub-rounds (the entries' vertices would need a third table).
+// A predecessor is the vertex of the position's entry, read from the frontier
+// for the winners only.
 template <int B, bool PRED, bool CULL = true, bool WHOLE = false>
 __device__ __forceinline__ void expand_range_warp(const BfsParams &p, const VertexFrontier &in,
                                                   ExpandSmem<B, PRED> &s, int level, const VertexFrontier &vout,
                                                   unsigned long long *qe_out, const EdgeFrontier *eout = nullptr,
                                                   unsigned long long skip_above = ~0ull)
 {
-    static_assert(B <= 256 || !PRED, "predecessor tables exist for CTAs of up to 256 threads only");
     constexpr int NW = B / 32;
     constexpr int PW = kWarpSlice / 32;    // positions per lane per slice
     constexpr int CAP = kChunkMax / NW;    // a warp's output entries
     // positions per lane per batch: with CTAs of more than 256 threads a warp's
     // output holds half a slice, so the slice goes in two halves, except with
     // WHOLE (top-down-only searches), which test the whole slice at once and
-    // append its winners in halves: expand-contract 888 -> 852 us per R-MAT 22
+    // append its winners in parts: expand-contract 888 -> 852 us per R-MAT 22
     // search, while direction-optimizing searches and the edge strategies'
     // copy pass measured 1-4% slower that way
     constexpr int PB = (CULL && WHOLE) || CAP / 32 >= PW ? PW : CAP / 32;
@@ -1094,7 +1055,6 @@ __device__ __forceinline__ void expand_range_warp(const BfsParams &p, const Vert
     int32_t *bd = s.rel + warp * CAP;
     uint16_t *own = s.wmap + warp * kWarpSlice;  // slice position -> table entry
     int32_t *tcol = s.wcol + warp * kWarpSlice;  // table entry -> column index of slice position 0
-    int32_t *tver = PRED ? s.vert + warp * kWarpSlice : nullptr;
     const int q = s.q, re = s.E;
     int count = 0;  // warp-uniform
     bool any = false;
@@ -1102,22 +1062,23 @@ __device__ __forceinline__ void expand_range_warp(const BfsParams &p, const Vert
     for (long long x64 = (long long)warp_slice0(warp) * kWarpSlice; x64 < re; x64 += stride) {
         const int x0 = (int)x64;
         const int len = min(kWarpSlice, re - x0);
-        warp_slice_map<PRED>(in, q, x0, len, own, tcol, tver);
+        const int i0 = warp_slice_map(in, q, x0, len, own, tcol);
 #pragma unroll
         for (int h = 0; h < PW / PB; h++) {
-            int v[PB], u[PB];
+            int v[PB];
             bool go[PB];
-            warp_slice_gather<PB, PRED>(p, h, len, own, tcol, tver, v, u, go);
+            warp_slice_gather<PB>(p, h, len, own, tcol, v, go);
+            const auto pred = [&](int t) { return ld_cg(in.v + i0 + own[(h * PB + t) * 32 + lane]); };
             if constexpr (CULL) {
-                any |= warp_discover<PB, PRED, true, CAP>(p, s.mask, v, u, go, level + 1, bv, bc, bd, count,
-                                                     vout, qe_out, skip_above);
+                any |= warp_discover<PB, PRED, true, CAP>(p, s.mask, v, go, level + 1, pred, bv, bc, bd, count, vout,
+                                                          qe_out, skip_above);
             } else {
 #pragma unroll
                 for (int t = 0; t < PB; t++) {
                     if (go[t]) {
                         const int r = (h * PB + t) * 32 + lane;
                         eout->v[x0 + r] = v[t];
-                        if (PRED) eout->pred[x0 + r] = u[t];
+                        if (PRED) eout->pred[x0 + r] = pred(t);
                     }
                 }
             }
@@ -2062,9 +2023,15 @@ template <int B, bool PRED>
 __device__ __forceinline__ void begin_pass(const BfsParams &p, ExpandSmem<B, PRED> &s, int pass, bool count_queue)
 {
     if (threadIdx.x == 0) {
+        // (independent loads, one round trip for all of them)
         const unsigned long long x = ld_cg64(&p.st->qe[pass % 3]);
+        const unsigned long long visited = ld_cg64(&p.st->visited_edges[pass % 3]);
+        const unsigned error = ld_cg(&p.st->error);
+        const int dir = ld_cg(&p.st->dir[pass % 3]), sel = ld_cg(&p.st->mask_sel[pass % 3]);
+        s.depth_limit = ld_cg(&p.st->depth_limit);
         s.q = qe_count(x);
         s.E = qe_edges(x);
+        s.error = error;
         s.flag = 0;
         if ((unsigned)s.E > (unsigned)p.edges || (unsigned)s.q > (unsigned)max(p.vcap, p.ecap)) {
             // counters past the graph's size: stop before any frontier read
@@ -2078,9 +2045,9 @@ __device__ __forceinline__ void begin_pass(const BfsParams &p, ExpandSmem<B, PRE
             // aggregates from iteration 1 on, contract_expand_atomic/kernel.cuh:333-345)
             if (count_queue && pass > 0) atomicAdd(&p.st->total_queued, (unsigned long long)s.q);
         }
-        s.visited_edges = ld_cg64(&p.st->visited_edges[pass % 3]) + (unsigned long long)s.E;
-        s.prev_bu = ld_cg(&p.st->dir[pass % 3]);
-        s.mask = ld_cg(&p.st->mask_sel[pass % 3]) ? p.mask_alt : p.mask;
+        s.visited_edges = visited + (unsigned long long)s.E;
+        s.prev_bu = dir;
+        s.mask = sel ? p.mask_alt : p.mask;
         s.ul_in = -1;
         s.ul_n = 0;
         if (p.ul[0]) {
@@ -2125,8 +2092,7 @@ __device__ __forceinline__ void record_direction(const BfsParams &p, unsigned lo
     if (bu && p.levels && pass < kMaxLevelRecords) p.levels[pass].bottom_up = 1;
 }
 
-// A phase of levels run by part of the grid (CTA 0 alone, or the first
-// kSubgridCtas CTAs) starts at a pass whose state slots (qe[pass % 3] and the
+// A phase of levels run by part of the grid (team_phase) starts at a pass whose state slots (qe[pass % 3] and the
 // direction slots) every CTA reads in begin_pass; the CTAs outside the phase
 // then wait at the grid barrier.  Block 0 reuses those slots two passes on, so
 // before its second level it waits (thread 0, bounded) until the `outside` CTAs
@@ -2140,27 +2106,313 @@ __device__ __forceinline__ void outside_arrived(const BfsParams &p, ExpandSmem<B
     __syncthreads();
 }
 
-constexpr int kSoloLevelCap = 4096;  // small levels CTA 0 runs alone before the grid resynchronises
+// ------------------------------------------------------------------------------------
+// Resident levels: a team of CTAs (one, or the first `team` of the grid) runs
+// top-down levels one after the other with each CTA's frontier in its own run
+// tables (n entries: rel = degree prefix with rel[n] = E, colstart = row start,
+// vert = vertex in predecessor searches).  The frontier arrays are read when the
+// phase starts, cut into equal shares of edges, and written when it ends; in
+// between a CTA expands what it found itself: owner map, gather, visited test
+// beside the CSR rows, and one CTA scan that places the winners in the same
+// tables.  One team barrier per level carries the sums that decide the next one
+// in its arrival word, so a level costs no frontier, counter or chunk-index
+// traffic and no read after the barrier.  A single CTA needs no barrier at all.
+// What bounds it: the round trips of the column indices, of the test and of the
+// barrier.  Lattice levels of 1000 to 8000 edges: 8.2 -> 3.9 us; of 60 to 250
+// thousand: 13 -> 5.6 us; levels under 256 edges on one CTA: 3.7 -> 2.0 us.
+// ------------------------------------------------------------------------------------
+constexpr int kTeamLevelCap = 4096;  // levels of a phase before the grid resynchronises
+constexpr int kTeamShare = 512;      // edges per CTA a team is sized for
+// A CTA whose next level passes this many edges ends the phase, and the next one
+// starts with equal shares again (a team of the whole grid uses its tables up).
+constexpr int kTeamFull = 1536;
+// the arrival word: CTAs arrived, CTAs too full, entries, edges (of the others)
+constexpr int kTeamArrive = 52, kTeamOver = 42, kTeamCount = 21;
+constexpr unsigned kTeamMask = (1u << 21) - 1u;
+constexpr int kTeamMaxCtas = (1 << 10) - 1;  // (each at most 2047 entries or 2048 edges: the sums fit 21 bits)
+
+__device__ __forceinline__ int team_limit(const BfsParams &p)
+{
+    return min(min((int)gridDim.x, p.team_edges > 0 ? kSubgridCtas : kTeamMaxCtas), kTeamMaxCtas);
+}
+
+// CTAs for a level of E edges (visited_edges: of the levels up to it), 0: the
+// level runs on the whole grid.  A level larger than all before it is likely to
+// be followed by a larger one, and a phase of one level only adds a barrier:
+// such levels form a team only where the graph's remaining edges fit one, and
+// the team is sized for them.
+__device__ __forceinline__ int team_size(const BfsParams &p, int E, unsigned long long visited_edges)
+{
+    const int most = team_limit(p);
+    if (p.team_edges < 0 || most < 2 || E > most * (kTeamShare * 2) || (p.team_edges > 0 && E > p.team_edges)) return 0;
+    if (2ull * (unsigned)E > visited_edges && p.team_edges == 0) {
+        const unsigned long long left = (unsigned long long)p.edges - min((unsigned long long)p.edges, visited_edges);
+        if (left > (unsigned long long)most * (kTeamShare * 2)) return 0;
+        E = max(E, (int)left / 2);
+    }
+    return max(2, min(most, (E + kTeamShare - 1) / kTeamShare));
+}
+
+// Barrier of the team with the sums of every CTA's `add` (below kTeamArrive)
+// left in s.team_sum; block 0 clears the slot two barriers on.  A wait that runs
+// out sets the error word and s.error.
+template <typename Smem>
+__device__ __forceinline__ void team_barrier(const BfsParams &p, Smem &s, int team, unsigned &seq,
+                                             unsigned long long add)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long *slot = &p.st->team[seq % 3];
+        red_release(slot, add + (1ull << kTeamArrive));
+        unsigned spins = 0;
+        unsigned long long x;
+        while ((int)((x = ld_acquire(slot)) >> kTeamArrive) < team) {
+            if (++spins > p.spin_limit) {
+                atomicOr(&p.st->error, kErrBarrier);
+                s.error = kErrBarrier;
+                break;
+            }
+            if ((spins & 15) == 0 && (s.error = ld_cg(&p.st->error)) != 0) break;
+            if (spins >= 64) __nanosleep(spins < 256 ? 64 : 256);
+        }
+        if (blockIdx.x == 0) p.st->team[(seq + 2) % 3] = 0;
+        s.team_sum = x & ((1ull << kTeamArrive) - 1ull);
+    }
+    seq++;
+    __syncthreads();
+}
+
+// Runs levels from `level` on; on return `level` is the first one not run, its
+// frontier is in the vertex frontier arrays and its state slots are set, as a
+// level run by the whole grid leaves them.  All threads of the team's CTAs call
+// it, after begin_pass; `limit`: largest level of a team of one; `generation`:
+// grid barriers passed; `seq`: team barriers passed.
+template <int B, bool PRED, bool LISTS, bool BU>
+__device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRED> &s, int &level, int team, int limit,
+                                           unsigned generation, unsigned &seq)
+{
+    constexpr int N = ExpandSmem<B, PRED>::kEntries;
+    constexpr int PER = N / B;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int dl = s.depth_limit, first = level;
+    const int full = team == 1 ? limit : team < team_limit(p) ? kTeamFull : N;
+    unsigned long long visited = s.visited_edges;  // through the level being run
+    unsigned long long queued = 0;
+    unsigned leaves = 0;
+    int last_found = -1;  // last level at which this thread labelled a vertex
+    int n = 0, E = 0;     // this CTA's share
+    {
+        const VertexFrontier in = p.vf[level & 1];
+        const int q = s.q;
+        int rs, re;
+        cta_range(s.E, blockIdx.x, team, rs, re);
+        if (rs < re) {
+            const int i0 = rs == 0 ? 0 : ld_cg(in.cf + rs / kChunkGrain);
+            E = re - rs;
+            for (int b = 0;; b += B) {
+                const int j = b + tid, i = i0 + j;
+                bool inside = false;
+                if (i < q && j < N) {
+                    const int Pi = ld_cg(in.P + i), ci = ld_cg(in.col + i);
+                    const int vi = PRED ? ld_cg(in.v + i) : 0;
+                    if (Pi < re) {
+                        inside = true;
+                        const int start = max(Pi, rs);
+                        s.rel[j] = start - rs;
+                        s.colstart[j] = ci + (start - Pi);
+                        if (PRED) s.vert[j] = vi;
+                    }
+                }
+                const int c = __syncthreads_count(inside);
+                n += c;
+                if (c < B) break;
+            }
+            if (tid == 0) s.rel[n] = E;
+        }
+    }
+    __syncthreads();
+    unsigned long long tot = 0;
+    // a level of more edges than the graph has vertices meets visited ones mostly,
+    // and on few mask words: its atomics alone would queue up (random 20,000
+    // vertices, 237 thousand edges: 33 us, with the pre-check 10)
+    bool precheck = p.precheck && s.E > p.nodes;
+    for (int run = 0;; run++) {
+        if (E > 0) stamp(p, level, 0);
+        fill_owners<B>(s, n);
+        __syncthreads();
+        int v[PER], u[PER];
+#pragma unroll
+        for (int t = 0; t < PER; t++) {
+            const int x = t * B + tid;
+            v[t] = u[t] = -1;
+            if (x < E) {
+                const int j = s.own[x];
+                v[t] = ld_stream(p.column_indices + s.colstart[j] + (x - s.rel[j]));
+                if (PRED) u[t] = s.vert[j];
+            }
+        }
+        // visited test, the rows beside it
+        int r0[PER], deg[PER];
+        unsigned found = 0;
+        if (LISTS && s.ul_in >= 0) {
+            // (bottom-up list mode gave up the mask: the labels decide)
+#pragma unroll
+            for (int t = 0; t < PER; t++) {
+                r0[t] = deg[t] = 0;
+                if (v[t] >= 0 && ld_cg(p.labels + v[t]) == -1 && atomicCAS(p.labels + v[t], -1, level + 1) == -1) {
+                    found |= 1u << t;
+                    r0[t] = ld_ro(p.row_offsets + v[t]);
+                    deg[t] = ld_ro(p.row_offsets + v[t] + 1);
+                }
+            }
+        } else {
+            if (precheck) {
+                unsigned word[PER];
+#pragma unroll
+                for (int t = 0; t < PER; t++) word[t] = v[t] >= 0 ? ld_cg(s.mask + (v[t] >> 5)) : 0u;
+#pragma unroll
+                for (int t = 0; t < PER; t++)
+                    if ((word[t] >> (v[t] & 31)) & 1u) v[t] = -1;
+            }
+            unsigned old[PER];
+#pragma unroll
+            for (int t = 0; t < PER; t++) {
+                old[t] = ~0u;
+                if (v[t] >= 0) old[t] = atomicOr(s.mask + (v[t] >> 5), 1u << (v[t] & 31));
+            }
+#pragma unroll
+            for (int t = 0; t < PER; t++) {
+                r0[t] = deg[t] = 0;
+                if (v[t] >= 0) {
+                    r0[t] = ld_ro(p.row_offsets + v[t]);
+                    deg[t] = ld_ro(p.row_offsets + v[t] + 1);
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < PER; t++)
+                if (!((old[t] >> (v[t] & 31)) & 1u)) found |= 1u << t;
+        }
+        unsigned cnt = 0;
+        unsigned long long sum = 0;
+#pragma unroll
+        for (int t = 0; t < PER; t++) {
+            const bool f = (found >> t) & 1u;
+            if (f) p.labels[v[t]] = PRED ? u[t] : level + 1;
+            deg[t] = f ? deg[t] - r0[t] : 0;
+            if (f && deg[t] == 0) leaves++;
+            if (deg[t] > 0) cnt++;
+            sum += (unsigned)deg[t];
+        }
+        level++;
+        if (found) last_found = level;
+        const unsigned long long at = cta_exclusive_scan<B>(((unsigned long long)cnt << 32) + sum, s.scan_warp, &tot);
+        unsigned g = (unsigned)(at >> 32), d = (unsigned)(at & 0xffffffffu);
+#pragma unroll
+        for (int t = 0; t < PER; t++) {
+            if (deg[t] > 0) {
+                s.colstart[g] = r0[t];
+                s.rel[g] = (int)d;
+                if (PRED) s.vert[g] = v[t];
+                g++;
+                d += (unsigned)deg[t];
+            }
+        }
+        n = qe_count(tot);
+        E = qe_edges(tot);
+        if (tid == 0) s.rel[n] = E;
+        // the whole next level: its entries and edges, and whether a CTA is too full
+        int n_all = n, E_all = E;
+        bool over = E > full;
+        if (team > 1) {
+            team_barrier(p, s, team, seq,
+                         over ? 1ull << kTeamOver
+                              : ((unsigned long long)(unsigned)n << kTeamCount) + (unsigned long long)(unsigned)E);
+            const unsigned long long x = s.team_sum;
+            E_all = (int)(x & kTeamMask);
+            n_all = (int)((x >> kTeamCount) & kTeamMask);
+            over = (x >> kTeamOver) != 0;
+        } else {
+            // (a wait that expired elsewhere ends the phase too: read now and then)
+            if (tid == 0 && (run & 63) == 63) s.error = ld_cg(&p.st->error);
+            __syncthreads();
+        }
+        // (a frontier larger than the queue goes out too, so the overflow is reported;
+        // a phase that has shrunk goes on with a smaller team)
+        if (over || n_all == 0 || n_all > p.vcap || (dl >= 0 && level >= dl) || run + 1 >= kTeamLevelCap ||
+            s.error != 0 || (team > 1 && run >= 8 && E_all < team * (kTeamShare / 8)) ||
+            (team > 1 && p.team_edges > 0 && E_all > p.team_edges) ||
+            (BU && team > 1 &&
+             choose_bottom_up(p, false, n_all, E_all, visited + (unsigned long long)(unsigned)E_all)))
+            break;
+        precheck = p.precheck && E_all > p.nodes;
+        visited += (unsigned long long)(unsigned)E_all;
+        queued += (unsigned long long)(unsigned)n_all;
+        if (run == 0 && blockIdx.x == 0) {
+            // the phase's input slot is an output slot again two levels on
+            outside_arrived(p, s, generation, gridDim.x - team);
+            if (tid == 0) p.st->qe[first % 3] = 0;
+        }
+        if (tid == 0 && blockIdx.x == 0 && p.levels && level < kMaxLevelRecords) {
+            LevelRecord r;
+            r.vertices = n_all;
+            r.edges = E_all;
+            r.bottom_up = 0;
+            r.pass = level;
+            r.t_ns = globaltimer_ns();
+            p.levels[level] = r;
+        }
+    }
+    leaves = __reduce_add_sync(0xffffffffu, leaves);
+    last_found = __reduce_max_sync(0xffffffffu, last_found);
+    if (lane == 0 && leaves) atomicAdd(&p.st->total_queued, (unsigned long long)leaves);
+    if (lane == 0 && last_found >= 0) atomicMax(&p.st->max_level, last_found);
+    if (tid == 0 && blockIdx.x == 0) {
+        record_direction(p, visited, level - 1, false, s.mask, s.ul_in, s.ul_n);
+        p.st->tile_ctr[level % 3] = 0;
+        if (p.ul[0]) p.st->ul_count[(level + 1) % 3] = 0;
+        if (queued) atomicAdd(&p.st->total_queued, queued);
+    }
+    if (n == 0) return;
+    // the last winners become the frontier of `level`
+    int dj[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int j = k * B + tid;
+        dj[k] = j < n ? s.rel[j + 1] - s.rel[j] : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int j = k * B + tid;
+        if (j < n) {
+            s.rel[j] = dj[k];
+            if (PRED) s.out[j] = s.vert[j];
+        }
+    }
+    if (tid == 0) s.out_count = n;
+    __syncthreads();
+    emit_frontier<B, PRED>(p, s, level - 1, p.vf[level & 1], &p.st->qe[level % 3], false);
+    __syncthreads();
+}
+
 // bottom-up levels emit their frontier (rather than count it) once the unvisited
 // edges are under 1 / kDeferMinShare of the graph's
 constexpr unsigned long long kDeferMinShare = 512;
 
 // Expand-contract (vertex frontiers): one level per pass.  With
-// direction_opt, levels with a large frontier run bottom-up.  In a
-// persistent launch, a run of levels whose frontiers have at most
-// p.small_edges edges is processed by CTA 0 alone, separated by CTA-level
-// barriers only, while the other CTAs wait at the grid barrier; while those
-// levels fit one sub-round their frontier stays in shared memory.
+// direction_opt, levels with a large frontier run bottom-up.  In a persistent
+// launch, runs of small and mid-size top-down levels are processed by a team of
+// CTAs that keep their frontiers in shared memory (team_phase), while the other
+// CTAs wait at the grid barrier.
 // BU = false builds a top-down-only variant (plain expand-contract searches):
 // without the bottom-up code the kernel needs fewer registers.
-template <int B, bool PRED, bool LISTS, bool SUBGRID = false, bool BU = true>
+template <int B, bool PRED, bool LISTS, bool BU = true>
 __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
 {
     // top-down levels with at least a full sub-round per CTA run warp by warp
-    // (expand_range_warp) when the policy asks for it (not in list mode, nor
-    // predecessor searches with CTAs of more than 256 threads)
+    // (expand_range_warp) when the policy asks for it (not in list mode)
     const auto warp_levels = [](const BfsParams &q, int E) {
-        return !LISTS && (B <= 256 || !PRED) && q.warp_contract != 0 && warp_sized(E);
+        return !LISTS && q.warp_contract != 0 && warp_sized(E);
     };
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ExpandSmem<B, PRED> &s = *reinterpret_cast<ExpandSmem<B, PRED> *>(smem_raw);
@@ -2173,22 +2425,22 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
     late_start(p);
     int level = ld_cg(&p.st->cur_level);
     bool limit_hit = false, worked = false;
-    int solo_phase = 0;  // small-frontier phases so far (the same count in every CTA)
-    int sub_phase = 0;   // sub-grid phases so far (the same count in every CTA)
-    unsigned sub_generation = 0;  // barriers of sub-grid phases this CTA took part in
+    int phase = 0;          // resident phases so far (the same count in every CTA)
+    unsigned team_seq = 0;  // team barriers so far in the search, as of the last phase's end
+    const int solo_edges = min(p.small_edges, ExpandSmem<B, PRED>::kEntries);  // largest level of one CTA
     DutyClock duty(p);
     __syncthreads();
     for (int iter = 0; iter < p.max_levels; iter++, level++) {
         int pass = level;
         begin_pass<B, PRED>(p, s, pass, true);
-        if (s.q == 0 || ld_cg(&p.st->error) != 0) break;
-        const int dl = p.st->depth_limit;
+        if (s.q == 0 || s.error != 0) break;
+        const int dl = s.depth_limit;
         if (dl >= 0 && level >= dl) {
             limit_hit = true;
             break;
         }
         if (BU && s.prev_bu == 2 &&
-            ((p.persistent && s.E <= p.small_edges) || !choose_bottom_up(p, true, s.q, s.E, s.visited_edges))) {
+            ((p.persistent && s.E <= solo_edges) || !choose_bottom_up(p, true, s.q, s.E, s.visited_edges))) {
             // the previous level ran bottom-up and only counted its discoveries:
             // this top-down level (or solo phase) reads them as a vertex frontier
             materialize_frontier<B, PRED>(p, s, p.vf[level & 1]);
@@ -2196,154 +2448,30 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
             if (tid == 0 && ld_cg64(&p.st->mat_ctr) != ld_cg64(&p.st->qe[pass % 3]))
                 atomicOr(&p.st->error, kErrFrontier);
         }
-        if (p.persistent && s.E <= p.small_edges) {
-            // ---- small frontiers: CTA 0 alone, level after level ----------------------
-            const int solo_pass = pass;  // (instrumented searches stamp the arrivals under it)
-            if (blockIdx.x == 0) {
-                int smem_n = -1;  // >= 0: this level's frontier is the run tables in shared memory (entries)
-                for (int solo = 0;; solo++) {
-                    if (tid == 0) record_direction(p, s.visited_edges, pass, false, s.mask, s.ul_in, s.ul_n);
-                    const bool one_round = s.E > 0 && s.E <= kChunkMax;  // CTA-uniform
-                    if (smem_n >= 0)
-                        solo_level_smem<B, PRED, LISTS>(p, s, level, smem_n, s.E);
-                    else
-                        expand_range<B, PRED, true, LISTS>(p, p.vf[level & 1], s, level, pass,
-                                                           p.vf[(level + 1) & 1], p.ef[0],
-                                                           &p.st->qe[(pass + 1) % 3], bar_phase, 0, 1, one_round);
-                    __syncthreads();
-                    if (s.flag) max_level_seen = level + 1;
-                    level++;
-                    pass = level;
-                    if (one_round) {
-                        // the discoveries are still in s.out / colstart / rel: stay in
-                        // shared memory while the next level is one sub-round too
-                        constexpr int PER = kChunkMax / B;
-                        const int n = s.out_count;
-                        int deg[PER];
-                        unsigned long long sum = 0;
-#pragma unroll
-                        for (int k = 0; k < PER; k++) {
-                            const int j = tid * PER + k;
-                            deg[k] = j < n ? s.rel[j] : 0;
-                            sum += (unsigned long long)deg[k];
-                        }
-                        unsigned long long En;
-                        unsigned long long run = cta_exclusive_scan<B>(sum, s.scan_warp, &En);
-                        // (a frontier larger than the queue goes out too, so the overflow is reported)
-                        if (tid == 0)
-                            s.solo_stop = n == 0 || n > p.vcap ||
-                                          En > (unsigned long long)min(p.small_edges, kChunkMax) ||
-                                          (dl >= 0 && level >= dl) || solo + 1 >= kSoloLevelCap ||
-                                          ld_cg(&p.st->error) != 0;
-                        __syncthreads();
-                        if (!s.solo_stop && solo == 0) outside_arrived(p, s, generation, gridDim.x - 1);
-                        if (!s.solo_stop) {
-#pragma unroll
-                            for (int k = 0; k < PER; k++) {
-                                const int j = tid * PER + k;
-                                if (j < n) {
-                                    s.rel[j] = (int)run;
-                                    if (PRED) s.vert[j] = s.out[j];
-                                }
-                                run += (unsigned long long)deg[k];
-                            }
-                            if (tid == 0) {
-                                // begin_pass without the frontier counters
-                                s.rel[n] = (int)En;
-                                s.q = n;
-                                s.E = (int)En;
-                                s.flag = 0;
-                                s.out_count = 0;
-                                s.visited_edges += En;
-                                p.st->qe[(pass + 2) % 3] = 0;
-                                p.st->tile_ctr[(pass + 1) % 3] = 0;
-                                atomicAdd(&p.st->total_queued, (unsigned long long)n);
-                                if (p.ul[0]) p.st->ul_count[(pass + 2) % 3] = 0;
-                                if (p.levels && pass < kMaxLevelRecords) {
-                                    LevelRecord r;
-                                    r.vertices = n;
-                                    r.edges = (int)En;
-                                    r.bottom_up = 0;
-                                    r.pass = pass;
-                                    r.t_ns = globaltimer_ns();
-                                    p.levels[pass] = r;
-                                }
-                            }
-                            smem_n = n;
-                            __syncthreads();
-                            continue;
-                        }
-                        // leaving shared memory: the discoveries become the frontier of `pass`
-                        emit_frontier<B>(p, s, pass - 1, p.vf[level & 1], &p.st->qe[pass % 3]);
-                        __syncthreads();
-                        smem_n = -1;
-                        // the phase ends here unless only the one-sub-round limit stopped it
-                        // (the frontier's size is known: no read of the counter it went to)
-                        if (n == 0 || En > (unsigned long long)p.small_edges || (dl >= 0 && level >= dl) ||
-                            solo + 1 >= kSoloLevelCap)
-                            break;
-                    }
-                    if (tid == 0) {
-                        const unsigned long long x = ld_cg64(&p.st->qe[pass % 3]);
-                        s.q = qe_count(x);
-                        s.E = qe_edges(x);
-                    }
-                    __syncthreads();
-                    const bool stop = s.q == 0 || s.E > p.small_edges || (dl >= 0 && level >= dl) ||
-                                      solo + 1 >= kSoloLevelCap || ld_cg(&p.st->error) != 0;
-                    if (stop) break;
-                    if (solo == 0) outside_arrived(p, s, generation, gridDim.x - 1);
-                    begin_pass<B, PRED>(p, s, pass, true);
+        // ---- small and mid-size top-down levels: a team of CTAs, level after level
+        int team = 0;
+        if (p.persistent) {
+            if (s.E <= solo_edges)
+                team = 1;
+            else if (!(BU && choose_bottom_up(p, s.prev_bu != 0, s.q, s.E, s.visited_edges)))
+                team = team_size(p, s.E, s.visited_edges);
+        }
+        if (team > 0) {
+            const int first = pass;  // (instrumented searches stamp the arrivals under it)
+            if ((int)blockIdx.x < team) {
+                team_phase<B, PRED, LISTS, BU>(p, s, level, team, team == 1 ? solo_edges : 0, generation, team_seq);
+                if (tid == 0 && blockIdx.x == 0) {
+                    p.st->phase_level[phase & 1] = level;
+                    p.st->phase_seq[phase & 1] = team_seq;
                 }
-                if (tid == 0) p.st->solo_resume[solo_phase & 1] = level;
             }
             worked = true;
-            stamp(p, solo_pass, kPhaseArrive);
+            stamp(p, first, kPhaseArrive);
             if (!duty.barrier(p.st, generation, &s_ok)) break;
             // not st->cur_level: CTA 0 may already have moved it on by the time a slow CTA reads
-            level = ld_cg(&p.st->solo_resume[solo_phase & 1]) - 1;  // the loop increment brings it back
-            solo_phase++;
-            continue;
-        }
-        // (a kernel variant of its own: the code would cost the other paths registers)
-        if (SUBGRID && p.persistent && p.subgrid_edges > 0 && s.E <= p.subgrid_edges &&
-            (int)gridDim.x >= 4 * kSubgridCtas &&
-            !(BU && choose_bottom_up(p, s.prev_bu != 0, s.q, s.E, s.visited_edges))) {
-            // ---- mid-size top-down levels: the first kSubgridCtas CTAs, level after
-            // level, with a barrier of their own; the others wait at the grid barrier
-            if ((int)blockIdx.x < kSubgridCtas) {
-                for (int sub = 0;; sub++) {
-                    if (tid == 0 && blockIdx.x == 0)
-                        record_direction(p, s.visited_edges, pass, false, s.mask, s.ul_in, s.ul_n);
-                    expand_range<B, PRED, true, LISTS>(p, p.vf[level & 1], s, level, pass, p.vf[(level + 1) & 1],
-                                                       p.ef[0], &p.st->qe[(pass + 1) % 3], bar_phase, blockIdx.x,
-                                                       kSubgridCtas);
-                    __syncthreads();
-                    if (s.flag) max_level_seen = level + 1;
-                    // (a wait that expires sets the error word: the test below then
-                    // ends the phase in every CTA of it)
-                    grid_barrier(&p.st->sub_barrier, sub_generation, &p.st->error, &s_ok, kSubgridCtas,
-                                 p.spin_limit);
-                    level++;
-                    pass = level;
-                    if (sub == 0 && blockIdx.x == 0) outside_arrived(p, s, generation, gridDim.x - kSubgridCtas);
-                    // the level's frontier is counted once, by the pass that processes it
-                    begin_pass<B, PRED>(p, s, pass, false);
-                    if (tid == 0)
-                        s.solo_stop = s.q == 0 || s.E > p.subgrid_edges || s.E <= p.small_edges ||
-                                      (dl >= 0 && level >= dl) || sub + 1 >= kSoloLevelCap ||
-                                      ld_cg(&p.st->error) != 0 ||
-                                      (BU && choose_bottom_up(p, s.prev_bu != 0, s.q, s.E, s.visited_edges));
-                    __syncthreads();
-                    if (s.solo_stop) break;
-                    if (tid == 0 && blockIdx.x == 0) atomicAdd(&p.st->total_queued, (unsigned long long)s.q);
-                }
-                if (tid == 0 && blockIdx.x == 0) p.st->sub_resume[sub_phase & 1] = level;
-            }
-            worked = true;
-            if (!duty.barrier(p.st, generation, &s_ok)) break;
-            level = ld_cg(&p.st->sub_resume[sub_phase & 1]) - 1;  // the loop increment brings it back
-            sub_phase++;
+            level = ld_cg(&p.st->phase_level[phase & 1]) - 1;  // the loop increment brings it back
+            team_seq = ld_cg(&p.st->phase_seq[phase & 1]);
+            phase++;
             continue;
         }
         const bool bu = BU && choose_bottom_up(p, s.prev_bu != 0, s.q, s.E, s.visited_edges);
@@ -2371,7 +2499,7 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
             bottom_up_windows<B, PRED>(p, s, level, pass, p.vf[(level + 1) & 1], &p.st->qe[(pass + 1) % 3], defer);
         else if (!BU && warp_levels(p, s.E))
         {
-            if constexpr (!BU && !LISTS && (B <= 256 || !PRED))
+            if constexpr (!BU && !LISTS)
                 expand_range_warp<B, PRED, true, true>(p, p.vf[level & 1], s, level, p.vf[(level + 1) & 1],
                                                        &p.st->qe[(pass + 1) % 3]);
         }
@@ -2388,16 +2516,16 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
                 const unsigned long long un =
                     (unsigned long long)p.edges - min((unsigned long long)p.edges, s.visited_edges);
                 skip_above = max(un / (unsigned long long)(p.bu_alpha + 1),
-                                 (unsigned long long)max(p.small_edges, 0));
+                                 (unsigned long long)max(solo_edges, 0));
             }
             if (BU && warp_levels(p, s.E)) {
-                if constexpr (BU && !LISTS && (B <= 256 || !PRED))
+                if constexpr (BU && !LISTS)
                     expand_range_warp<B, PRED>(p, p.vf[level & 1], s, level, p.vf[(level + 1) & 1],
                                                &p.st->qe[(pass + 1) % 3], nullptr, skip_above);
             } else {
                 expand_range<B, PRED, true, LISTS>(p, p.vf[level & 1], s, level, pass, p.vf[(level + 1) & 1],
                                                    p.ef[0], &p.st->qe[(pass + 1) % 3], bar_phase, blockIdx.x,
-                                                   gridDim.x, false, skip_above);
+                                                   gridDim.x, skip_above);
             }
         }
         __syncthreads();
@@ -2453,7 +2581,7 @@ __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
         if (p.phase_mask & 1) {
             const int pass = 2 * level;
             begin_pass<B, PRED>(p, s, pass, false);
-            if (ld_cg(&p.st->error) != 0 || s.q == 0) break;
+            if (s.error != 0 || s.q == 0) break;
             if (p.hybrid && p.persistent && s.q > (int)gridDim.x * p.saturation) {
                 saturated = true;  // the two-phase launches take this pass over (and count it)
                 break;
@@ -2471,7 +2599,7 @@ __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
                 if (!duty.barrier(p.st, generation, &s_ok)) break;
             }
         }
-        const int dl = p.st->depth_limit;
+        const int dl = (p.phase_mask & 1) ? s.depth_limit : p.st->depth_limit;
         if (dl >= 0 && level >= dl) {
             limit_hit = true;
             break;
@@ -2486,9 +2614,8 @@ __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
             }
             if (tid == 0 && blockIdx.x == 0) p.st->qe[(pass + 1) % 3] = pack((unsigned)(q == 0 ? 0 : E), 0u);
             if (q > 0) {
-                if ((B <= 256 || !PRED) && p.warp_contract && warp_sized(E)) {
-                    if constexpr (B <= 256 || !PRED)
-                        expand_range_warp<B, PRED, false>(p, p.vf[0], s, level, p.vf[1], nullptr, &p.ef[out_idx]);
+                if (p.warp_contract && warp_sized(E)) {
+                    expand_range_warp<B, PRED, false>(p, p.vf[0], s, level, p.vf[1], nullptr, &p.ef[out_idx]);
                 } else {
                     expand_range<B, PRED, false>(p, p.vf[0], s, level, pass, p.vf[1], p.ef[out_idx], nullptr,
                                                  bar_phase, blockIdx.x, gridDim.x);
@@ -2582,7 +2709,7 @@ __global__ void init_kernel(BfsParams p)
         st->cur_level = 0;
         st->epoch += 1ull << 24;
         st->barrier = 0;
-        st->sub_barrier = 0;
+        st->team[0] = st->team[1] = st->team[2] = 0;
         st->error = 0;
         st->max_level = 0;
         st->done = 0;

@@ -63,18 +63,17 @@ struct alignas(128) SearchState {
     int32_t dir[3];            // 1: the previous level ran bottom-up, 2: bottom-up with its frontier deferred
     int32_t mask_sel[3];       // which visited-mask buffer holds the visited set (0: mask, 1: mask_alt)
     unsigned long long visited_edges[3];  // degree sum of the vertices visited before the pass
-    // level at which a persistent launch resumes after a small-frontier phase of
-    // CTA 0, by phase parity (a slot is rewritten only two phases later, after
-    // every CTA has read it)
-    int32_t solo_resume[2];
-    // the same for a phase of mid-size top-down levels run by the first
-    // kSubgridCtas CTAs alone
-    int32_t sub_resume[2];
+    // level at which a persistent launch resumes after a resident phase, and the
+    // team barriers passed by then, by phase parity (a slot is rewritten only two
+    // phases later, after every CTA has read it)
+    int32_t phase_level[2];
+    uint32_t phase_seq[2];
     // slots of a deferred bottom-up frontier built at the start of the next
     // level (count << 32 | edge total; cleared when the bottom-up level starts)
     unsigned long long mat_ctr;
-    // arrival counter of the barrier among the CTAs of a sub-grid phase (its own line)
-    alignas(128) unsigned long long sub_barrier;
+    // a team's barriers, rotating by barrier % 3 (their own line): arrivals and the
+    // sums that decide the next level, in one word (team_phase)
+    alignas(128) unsigned long long team[3];
 };
 
 __host__ __device__ inline int qe_count(unsigned long long x) { return (int)(x >> 32); }
@@ -155,8 +154,9 @@ struct BfsParams {
     int32_t bu_alpha;         // switch to bottom-up when frontier edges > unvisited edges / alpha
     int32_t bu_beta;          // switch back to top-down when frontier vertices < n / beta
     int32_t small_edges;      // persistent launches: frontiers with at most this many edges run on CTA 0 alone
-    int32_t subgrid_edges;    // persistent launches: top-down frontiers with more than small_edges and at most
-                              // this many edges run on the first kSubgridCtas CTAs alone (0: off)
+    int32_t team_edges;       // persistent launches, top-down levels of more than small_edges edges: > 0 at most
+                              // this many run on a team of up to kSubgridCtas CTAs, 0 a team of any size,
+                              // < 0 never a team
     int32_t bu_scan;          // bottom-up continuation: 1 per lane, 2 per CTA (edge-parallel worklist)
     int32_t bu_long;          // bottom-up: lists longer than this are searched by the whole warp
     int32_t hist_log;         // history cull table of 2^hist_log entries per CTA (0: off)

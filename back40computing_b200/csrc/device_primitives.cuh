@@ -155,6 +155,12 @@ __device__ __forceinline__ void st_release(unsigned long long *p, unsigned long 
 {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+// release-add without a result: one instruction orders the CTA's writes (a CTA
+// barrier before it) and arrives
+__device__ __forceinline__ void red_release(unsigned long long *p, unsigned long long v)
+{
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ void st_relaxed(unsigned long long *p, unsigned long long v)
 {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -193,8 +199,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long *counter, unsign
     if (threadIdx.x == 0) {
         generation++;
         const unsigned long long target = (unsigned long long)generation * (count ? count : gridDim.x);
-        __threadfence();
-        atomicAdd(counter, 1ull);
+        red_release(counter, 1ull);
         unsigned spins = 0;
         int ok = 1;
         while (ld_acquire(counter) < target) {
@@ -203,13 +208,14 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long *counter, unsign
                 ok = 0;
                 break;
             }
-            if ((spins & 7) == 0 && ld_cg(error_word) != 0) {
+            if ((spins & 15) == 0 && ld_cg(error_word) != 0) {
                 ok = 0;
                 break;
             }
-            __nanosleep(spins < 64 ? 32 : 256);
+            // the first polls follow one another (a level's barrier is a few round
+            // trips long); only a long wait backs off
+            if (spins >= 64) __nanosleep(spins < 256 ? 64 : 256);
         }
-        __threadfence();
         *s_flag = ok;
     }
     __syncthreads();

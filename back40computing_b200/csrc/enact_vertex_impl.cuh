@@ -29,26 +29,17 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
     // distance searches with unvisited lists run the kernel variant that
     // carries list mode; the others keep the leaner code
     const bool lists_kernel = direction_opt && !PRED && pol.bottom_up_list > 0;
-    // fused searches with a sub-grid threshold run the variant that carries the
-    // sub-grid phase (not combined with list mode)
-    const bool subgrid_kernel = !lists_kernel && mode == B40C_ENACT_FUSED && pol.subgrid_frontier_edges > 0;
     // plain expand-contract searches (and directed graphs) never go bottom-up:
-    // they run the top-down-only variants; list mode and the sub-grid phase are
-    // built for 256-thread CTAs only
-    const void *kern = nullptr;
-    if (lists_kernel || subgrid_kernel) {
-        if constexpr (B == 256) {
-            kern = lists_kernel    ? (const void *)dev::ec_kernel<256, false, true>
-                   : direction_opt ? (const void *)dev::ec_kernel<256, PRED, false, true>
-                                   : (const void *)dev::ec_kernel<256, PRED, false, true, false>;
-        } else {
-            return b40c::fail(B40C_ERROR_INVALID_VALUE,
-                              "policy.threads %d: bottom-up list mode and the sub-grid phase need 256", B);
-        }
-    } else {
-        kern = direction_opt ? (const void *)dev::ec_kernel<B, PRED, false>
-                             : (const void *)dev::ec_kernel<B, PRED, false, false, false>;
-    }
+    // they run the top-down-only variants; list mode is built for 256-thread CTAs
+    // only, and a sub-grid threshold asks for them too
+    const bool subgrid = mode == B40C_ENACT_FUSED && pol.subgrid_frontier_edges > 0;
+    if (B != 256 && (lists_kernel || subgrid))
+        return b40c::fail(B40C_ERROR_INVALID_VALUE,
+                          "policy.threads %d: bottom-up list mode and the sub-grid phase need 256", B);
+    const void *kern = direction_opt ? (const void *)dev::ec_kernel<B, PRED, false>
+                                     : (const void *)dev::ec_kernel<B, PRED, false, false>;
+    if constexpr (B == 256)
+        if (lists_kernel) kern = (const void *)dev::ec_kernel<256, false, true>;
     const size_t smem = kernel_smem<dev::ExpandSmem<B, PRED>>(pol);
     int grid = 0;
     if ((rc = persistent_grid(p, kern, pol, max_grid, smem, &grid))) return rc;

@@ -41,6 +41,7 @@ struct MsParams {
 
 template <int B>
 struct MsSmem {
+    static constexpr int kEntries = kChunkMax;
     int32_t colstart[kChunkMax + 2];
     int32_t rel[kChunkMax + 2];
     unsigned long long fm[kChunkMax + 2];  // frontier mask of run j's vertex

@@ -148,7 +148,7 @@ BfsParams make_params(b40c_bfs_problem *p, const b40c_bfs_policy &pol)
     k.bu_beta = pol.bottom_up_beta;
     k.mask_alt = p->d_next;
     k.small_edges = pol.small_frontier_edges;
-    k.subgrid_edges = pol.subgrid_frontier_edges > 0 ? pol.subgrid_frontier_edges : 0;
+    k.team_edges = pol.subgrid_frontier_edges;
     k.bu_scan = pol.bottom_up_scan;
     k.bu_long = pol.bottom_up_long_list;
     k.hist_log = pol.history_cull > 0 ? kHistLog : 0;
@@ -182,7 +182,7 @@ b40c_bfs_policy default_policy(int strategy)
     pol.bottom_up_hub_probes = 1;
     pol.bottom_up_list = -1;
     pol.bottom_up_defer_frontier = 1;
-    pol.subgrid_frontier_edges = -1;
+    pol.subgrid_frontier_edges = 0;
     pol.bottom_up_long_list = 256;
     pol.history_cull = -1;
     pol.queue_allocation = 2;  // measured faster than look-back on RMAT-22 (1.75 vs 2.29 ms)
@@ -932,12 +932,11 @@ int b40c_bfs_enact_limited(b40c_bfs_problem *p, int strategy, int mode, int32_t 
     int rc = resolve_policy(strategy, policy, &pol);
     if (rc) return rc;
     // A caller that passes no policy at all (the reference's enactor calls)
-    // gets 512-thread CTAs for the distance searches of the top-down
-    // strategies: measured 2-10% faster than 256 threads on R-MAT 22, random
-    // 2^21, grid2d-1000 and grid3d-256 (hybrid with its hand-off scaled to the
-    // CTA size, enact_edge.cu).  Predecessor searches keep 256: their
-    // warp-by-warp levels need CTAs of at most 256 threads.
-    if (!policy && !p->mark_pred &&
+    // gets 512-thread CTAs for the top-down strategies: measured 2-10% faster
+    // than 256 threads on R-MAT 22, random 2^21, grid2d-1000 and grid3d-256
+    // (hybrid with its hand-off scaled to the CTA size, enact_edge.cu), and
+    // predecessor searches on R-MAT 20 340 -> 285 us.
+    if (!policy &&
         (strategy == B40C_EXPAND_CONTRACT || strategy == B40C_CONTRACT_EXPAND || strategy == B40C_TWO_PHASE ||
          strategy == B40C_HYBRID))
         pol.threads = 512;

@@ -121,9 +121,12 @@ typedef struct b40c_bfs_policy {
                                       from the two visited-mask buffers only when a top-down level
                                       follows: 1 = on (default), -1 = off */
     int32_t subgrid_frontier_edges; /* fused searches: runs of top-down levels with more than
-                                      small_frontier_edges and at most this many edges run on 16 CTAs
-                                      with a barrier of their own while the rest of the grid waits (the
-                                      mid-size levels of high-diameter graphs); -1 = off (default) */
+                                      small_frontier_edges edges run on a team of CTAs with a barrier of
+                                      their own, their frontier kept in shared memory, while the rest of
+                                      the grid waits (the mid-size levels of high-diameter graphs):
+                                      0 = levels of up to 1024 edges per CTA of the grid, on as many CTAs
+                                      as they need (default); > 0 = levels of at most this many edges, on
+                                      at most 16 CTAs (256-thread CTAs); -1 = off */
     int32_t bottom_up_long_list;   /* bottom-up levels: a vertex whose list is longer than this (and whose
                                       first probes found no parent) is searched by its whole warp, 32
                                       neighbours at a time; shorter lists are scanned by one lane, four at
@@ -140,9 +143,8 @@ typedef struct b40c_bfs_policy {
     int32_t warp_contract;         /* levels with at least a full 2048-edge sub-round per CTA, warp by warp:
                                       the contract and expand passes of the edge-frontier strategies
                                       (contract-expand, two-phase, hybrid), the top-down levels of
-                                      expand-contract and direction-optimizing searches (predecessor
-                                      searches: CTAs of up to 256 threads), and the pull levels of
-                                      batched searches.  1 = each warp works through its own slices of
+                                      expand-contract and direction-optimizing searches, and the pull
+                                      levels of batched searches.  1 = each warp works through its own slices of
                                       the level, dealt over every warp of the grid, with no CTA barriers,
                                       and sends its winners to the vertex frontier in flushes of its own
                                       (one packed atomic each; default), -1 = CTA-wide sub-rounds
