@@ -1938,13 +1938,17 @@ __device__ __forceinline__ void bottom_up_list(const BfsParams &p, ExpandSmem<B,
 // Direction of a level from the frontier's size (Beamer, Asanovic and
 // Patterson, SC'12 heuristic): top-down -> bottom-up when the frontier's
 // edges exceed the unvisited edges / alpha, bottom-up -> top-down when the
-// frontier falls under n / beta vertices.
+// frontier falls under n / beta vertices.  A bottom-up level reads the whole
+// visited mask, so a frontier of fewer than n / beta edges stays top-down
+// however few edges are left (the last levels of grid3d-201 went back and forth
+// between 5 us top-down and 60-90 us bottom-up levels: 3.54 -> 2.54 ms).
 __device__ __forceinline__ bool choose_bottom_up(const BfsParams &p, bool was_bottom_up, int q, int E,
                                                  unsigned long long visited_edges)
 {
     if (!p.direction_opt) return false;
     const long long unvisited_edges = (long long)p.edges - (long long)visited_edges;
-    if (!was_bottom_up) return (long long)E * p.bu_alpha > unvisited_edges;
+    if (!was_bottom_up)
+        return (long long)E * p.bu_alpha > unvisited_edges && (long long)E * p.bu_beta >= (long long)p.nodes;
     return (long long)q * p.bu_beta >= (long long)p.nodes;
 }
 
@@ -2509,14 +2513,15 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
             // E* * (alpha + 1) > the edges unvisited after this level's input, the
             // next level runs bottom-up whatever the rest adds (the switch test is
             // E * alpha > m - visited - E), so later tiles need not write entries.
-            // E* is at least the solo-phase threshold: a next level that small runs
-            // top-down on CTA 0 before any switch test.
+            // E* is at least the solo-phase threshold (a next level that small runs
+            // top-down on CTA 0 before any switch test) and the n / beta edges that
+            // the switch asks for.
             unsigned long long skip_above = ~0ull;
             if (BU && p.direction_opt && !LISTS) {
                 const unsigned long long un =
                     (unsigned long long)p.edges - min((unsigned long long)p.edges, s.visited_edges);
                 skip_above = max(un / (unsigned long long)(p.bu_alpha + 1),
-                                 (unsigned long long)max(solo_edges, 0));
+                                 (unsigned long long)max(max(solo_edges, 0), p.nodes / p.bu_beta));
             }
             if (BU && warp_levels(p, s.E)) {
                 if constexpr (BU && !LISTS)

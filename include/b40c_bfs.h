@@ -99,7 +99,8 @@ typedef struct b40c_bfs_policy {
     int32_t bottom_up_alpha;       /* direction-optimizing: go bottom-up when frontier edges exceed
                                       unvisited edges / alpha */
     int32_t bottom_up_beta;        /* direction-optimizing: return top-down when the frontier holds fewer
-                                      than nodes / beta vertices */
+                                      than nodes / beta vertices; go bottom-up only from a frontier of at
+                                      least nodes / beta edges */
     int32_t small_frontier_edges;  /* fused searches: runs of levels whose frontier has at most this many
                                       edges are processed by one CTA alone (CTA-level barriers only);
                                       -1 disables */
