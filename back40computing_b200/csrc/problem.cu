@@ -254,6 +254,29 @@ int resolve_policy(int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *out
     return B40C_SUCCESS;
 }
 
+// CTA size and CTAs per SM of a search whose caller left them open (no policy,
+// or 0 in it), each where it measured fastest (us per search):
+//  * 512 threads: against 256, R-MAT 22 direction-optimizing 135 / 119, R-MAT 20
+//    expand-contract 277 / 235 and its predecessors 330 / 272, R-MAT 16 73 / 63,
+//    grid3d-201 3900 / 3540 (list mode and a sub-grid threshold need 256);
+//  * one CTA per SM while the graph is small, where a level's cost is its barriers:
+//    direction-optimizing searches up to 2^19 vertices (R-MAT 16 63 / 55, R-MAT
+//    19 69 / 64, but random 10^6 112 / 130), top-down ones up to 2^21 edges
+//    (R-MAT 13 and random 20,000 107 / 67 and 100 / 62, R-MAT 17 88 / 92).
+void default_launch(const b40c_bfs_problem *p, int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *pol)
+{
+    if ((!in || in->threads == 0) && pol->bottom_up_list <= 0 && pol->subgrid_frontier_edges <= 0) {
+        pol->threads = 512;
+        // as resolve_policy gives the prefetch for a caller's 512
+        if (!in || in->bottom_up_prefetch == 0) pol->bottom_up_prefetch = pol->warp_bottom_up < 0 ? 1 : -1;
+    }
+    if (!in || in->ctas_per_sm == 0) {
+        const bool small = strategy == B40C_DIRECTION_OPTIMIZING ? p->nodes <= (int64_t)1 << 19
+                                                                 : p->edges <= (int64_t)1 << 21;
+        if (small && pol->threads == 512) pol->ctas_per_sm = 1;
+    }
+}
+
 // Device bytes a handle holds right now (the sizes its allocations asked
 // for; alloc_dev asks for at least 16 bytes).
 int64_t device_bytes(const b40c_bfs_problem *p)
@@ -931,15 +954,7 @@ int b40c_bfs_enact_limited(b40c_bfs_problem *p, int strategy, int mode, int32_t 
     b40c_bfs_policy pol;
     int rc = resolve_policy(strategy, policy, &pol);
     if (rc) return rc;
-    // A caller that passes no policy at all (the reference's enactor calls)
-    // gets 512-thread CTAs for the top-down strategies: measured 2-10% faster
-    // than 256 threads on R-MAT 22, random 2^21, grid2d-1000 and grid3d-256
-    // (hybrid with its hand-off scaled to the CTA size, enact_edge.cu), and
-    // predecessor searches on R-MAT 20 340 -> 285 us.
-    if (!policy &&
-        (strategy == B40C_EXPAND_CONTRACT || strategy == B40C_CONTRACT_EXPAND || strategy == B40C_TWO_PHASE ||
-         strategy == B40C_HYBRID))
-        pol.threads = 512;
+    default_launch(p, strategy, policy, &pol);
     DeviceGuard guard(p->device);
     p->timed = false;
     switch (strategy) {
