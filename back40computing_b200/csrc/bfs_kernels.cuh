@@ -2342,7 +2342,7 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
         }
         // (a frontier larger than the queue goes out too, so the overflow is reported;
         // a phase that has shrunk goes on with a smaller team)
-        if (over || n_all == 0 || n_all > p.vcap || (dl >= 0 && level >= dl) || run + 1 >= kTeamLevelCap ||
+        if (over || n_all == 0 || n_all > p.vcap || E_all > p.edge_limit || (dl >= 0 && level >= dl) || run + 1 >= kTeamLevelCap ||
             s.error != 0 || (team > 1 && run >= 8 && E_all < team * (kTeamShare / 8)) ||
             (team > 1 && p.team_edges > 0 && E_all > p.team_edges) ||
             (BU && team > 1 &&
@@ -2441,6 +2441,10 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
         const int dl = s.depth_limit;
         if (dl >= 0 && level >= dl) {
             limit_hit = true;
+            break;
+        }
+        if (s.E > p.edge_limit) {
+            if (tid == 0) atomicOr(&p.st->error, kErrOverflow);
             break;
         }
         if (BU && s.prev_bu == 2 &&
@@ -2558,101 +2562,65 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
     }
 }
 
-// Edge strategies: per level, contract the edge frontier into vf[0] (pass
-// 2L), then expand vf[0] into the next edge frontier at flattened edge
-// positions (pass 2L+1).  phase_mask selects the phases of a non-persistent
-// launch; a persistent launch runs both with a grid barrier after each.
-// With `hybrid`, a persistent launch returns when the edge frontier exceeds
-// gridDim * saturation items (SATURATION_QUIT, enactor_hybrid.cuh:571).
+// Edge strategies' per-level launches: contract the edge frontier into vf[0]
+// (pass 2L), then expand vf[0] into the next edge frontier at flattened edge
+// positions (pass 2L+1); phase_mask selects the launch's phase.
 template <int B, bool PRED>
 __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ExpandSmem<B, PRED> &s = *reinterpret_cast<ExpandSmem<B, PRED> *>(smem_raw);
-    __shared__ int s_ok;
     const int tid = threadIdx.x;
     if (tid == 0) mbar_init(&s.bar, 1);
     hist_init<B, PRED>(p, s, smem_raw);
-    unsigned bar_phase = 0, generation = 0;
+    unsigned bar_phase = 0;
     int max_level_seen = -1;
-    late_start(p);
-    int level = ld_cg(&p.st->cur_level);
-    bool limit_hit = false, saturated = false, completed_level = false;
+    const int level = ld_cg(&p.st->cur_level);
+    bool limit_hit = false, completed_level = false;
+    const int in_idx = p.edge_pingpong ? (level & 1) : 0;
+    const int out_idx = p.edge_pingpong ? ((level + 1) & 1) : 0;
     DutyClock duty(p);
     __syncthreads();
-    for (int iter = 0; iter < p.max_levels; iter++, level++) {
-        const int in_idx = p.edge_pingpong ? (level & 1) : 0;
-        const int out_idx = p.edge_pingpong ? ((level + 1) & 1) : 0;
-        if (p.phase_mask & 1) {
-            const int pass = 2 * level;
-            begin_pass<B, PRED>(p, s, pass, false);
-            if (s.error != 0 || s.q == 0) break;
-            if (p.hybrid && p.persistent && s.q > (int)gridDim.x * p.saturation) {
-                saturated = true;  // the two-phase launches take this pass over (and count it)
-                break;
-            }
+    if (p.phase_mask & 1) {
+        const int pass = 2 * level;
+        begin_pass<B, PRED>(p, s, pass, false);
+        if (s.error == 0 && s.q > 0) {
             if (tid == 0 && blockIdx.x == 0 && pass > 0) atomicAdd(&p.st->total_queued, (unsigned long long)s.q);
             if (p.warp_contract && warp_sized(s.q))
                 contract_range_warp<B, PRED>(p, s, p.ef[in_idx], level, p.vf[0], &p.st->qe[(pass + 1) % 3]);
             else
                 contract_range<B, PRED>(p, s, p.ef[in_idx], level, pass, &p.st->qe[(pass + 1) % 3]);
             __syncthreads();
-            if (s.flag) max_level_seen = max(max_level_seen, level);
-            if (p.persistent) {
-                if ((int)blockIdx.x == p.skip_arrival_cta)
-                    return;  // test-only: never arrives, so the others' bounded waits must run out
-                if (!duty.barrier(p.st, generation, &s_ok)) break;
-            }
+            if (s.flag) max_level_seen = level;
         }
-        const int dl = (p.phase_mask & 1) ? s.depth_limit : p.st->depth_limit;
-        if (dl >= 0 && level >= dl) {
-            limit_hit = true;
-            break;
-        }
-        if (p.phase_mask & 2) {
+    } else {
+        const int dl = p.st->depth_limit;
+        limit_hit = dl >= 0 && level >= dl;
+        if (!limit_hit) {
             const int pass = 2 * level + 1;
             begin_pass<B, PRED>(p, s, pass, false);
             const int q = s.q, E = s.E;
             if (E > p.ecap) {
                 if (tid == 0) atomicOr(&p.st->error, kErrOverflow);
-                break;
-            }
-            if (tid == 0 && blockIdx.x == 0) p.st->qe[(pass + 1) % 3] = pack((unsigned)(q == 0 ? 0 : E), 0u);
-            if (q > 0) {
-                if (p.warp_contract && warp_sized(E)) {
-                    expand_range_warp<B, PRED, false>(p, p.vf[0], s, level, p.vf[1], nullptr, &p.ef[out_idx]);
-                } else {
-                    expand_range<B, PRED, false>(p, p.vf[0], s, level, pass, p.vf[1], p.ef[out_idx], nullptr,
-                                                 bar_phase, blockIdx.x, gridDim.x);
+            } else {
+                if (tid == 0 && blockIdx.x == 0) p.st->qe[(pass + 1) % 3] = pack((unsigned)(q == 0 ? 0 : E), 0u);
+                if (q > 0) {
+                    if (p.warp_contract && warp_sized(E))
+                        expand_range_warp<B, PRED, false>(p, p.vf[0], s, level, p.vf[1], nullptr, &p.ef[out_idx]);
+                    else
+                        expand_range<B, PRED, false>(p, p.vf[0], s, level, pass, p.vf[1], p.ef[out_idx], nullptr,
+                                                     bar_phase, blockIdx.x, gridDim.x);
                 }
-            }
-            __syncthreads();
-            completed_level = true;
-            if (p.persistent) {
-                if (!duty.barrier(p.st, generation, &s_ok)) break;
-                // after the barrier, as in ec_kernel: late-starting CTAs read cur_level
-                if (tid == 0 && blockIdx.x == 0) p.st->cur_level = level + 1;
+                __syncthreads();
+                completed_level = true;
             }
         }
-        if (!p.persistent) break;
     }
     if (tid == 0 && max_level_seen >= 0) atomicMax(&p.st->max_level, max_level_seen);
     duty.finish();
-    if (p.persistent) {
-        if (tid == 0 && blockIdx.x == 0) {
-            p.st->cur_level = level;
-            if (saturated)
-                p.st->saturated = 1;
-            else
-                p.st->done = 1;
-        }
-    } else if (completed_level || limit_hit) {
-        finish_launch(p, level, 2 * (level + 1), limit_hit);
-    } else if (p.phase_mask & 2) {
-        // an expand launch that broke out (overflow, error) stops the search; a
-        // contract-only launch leaves the level's epilogue to its expand launch
-        finish_launch(p, level, 2 * (level + 1), false, true);
-    }
+    // the expand launch ends the level; one that broke out (overflow, error) stops
+    // the search
+    if (p.phase_mask & 2) finish_launch(p, level, 2 * (level + 1), limit_hit, !(completed_level || limit_hit));
 }
 
 // Sets up a search: the source's label, visited bit and the level-0
@@ -2718,7 +2686,6 @@ __global__ void init_kernel(BfsParams p)
         st->error = 0;
         st->max_level = 0;
         st->done = 0;
-        st->saturated = 0;
         st->total_queued = 0;
         st->finished = 0;
         st->qe[1] = st->qe[2] = 0;

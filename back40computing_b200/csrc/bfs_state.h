@@ -54,7 +54,6 @@ struct alignas(128) SearchState {
     unsigned long long epoch;  // look-back epoch base for this search
     int32_t max_level;         // deepest level at which a vertex was labelled
     int32_t done;              // 1 once the frontier emptied (or the depth limit was hit)
-    int32_t saturated;         // 1 when a hybrid fused launch handed off
     unsigned long long total_queued;  // sum of processed frontier lengths
     int32_t src;               // source vertex (read by the init kernel)
     int32_t depth_limit;       // < 0: unlimited
@@ -127,6 +126,8 @@ struct BfsParams {
     int32_t mask_words;
     int32_t vcap;  // vertex frontier capacity (entries)
     int32_t ecap;  // edge frontier capacity (entries)
+    int32_t edge_limit;  // largest level (edges) the search accepts: the edge frontiers' capacity of the
+                         // edge-frontier strategies, whose fused searches keep none
     int32_t max_chunks;
     int32_t cf_cap;  // entries of each vertex frontier's cf array (a level's edge total / kChunkGrain + 2)
     VertexFrontier vf[2];
@@ -139,7 +140,6 @@ struct BfsParams {
     int32_t cta_thresh;
     int32_t warp_cull;
     int32_t precheck;
-    int32_t saturation;       // hybrid: leave the fused kernel when items > gridDim * saturation
     int32_t persistent;       // 1: loop over levels with the grid barrier
     int32_t skip_arrival_cta; // test-only fault injection: this CTA never arrives (-1 = off)
     uint32_t late_start_ns;   // test-only: CTAs other than 0 of a persistent launch start this late (0 = off)
@@ -147,8 +147,7 @@ struct BfsParams {
     int32_t bulk_ok;          // 1: a sub-round inside one adjacency list may be staged by cp.async.bulk
                               // (column_indices is device memory; 0 for a host-mapped CSR)
     int32_t edge_pingpong;    // edge strategies: 1 = two edge frontiers (EDGE_FRONTIERS), 0 = one (MIXED)
-    int32_t phase_mask;       // edge kernel: 1 = contract, 2 = expand, 3 = both per level (persistent)
-    int32_t hybrid;           // edge kernel: leave the persistent loop when the frontier saturates
+    int32_t phase_mask;       // edge kernel: 1 = contract, 2 = expand
     int32_t alloc_lookback;   // 1: frontier slots by decoupled look-back, 0: one atomic per tile
     int32_t direction_opt;    // 1: levels may run bottom-up (symmetric graphs only)
     int32_t bu_alpha;         // switch to bottom-up when frontier edges > unvisited edges / alpha

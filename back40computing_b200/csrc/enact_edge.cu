@@ -1,7 +1,18 @@
 // Edge-frontier enactors: contract-expand (two O(m) edge frontiers), two-phase
-// (one O(n) vertex and one O(m) edge frontier) and hybrid (fused
-// contract-expand while the frontier is small, two-phase launches while it is
-// saturated; EnactorHybrid::EnactSearch, enactor_hybrid.cuh:279-551).
+// (one O(n) vertex and one O(m) edge frontier) and hybrid
+// (enactor_contract_expand.cuh:61, enactor_two_phase.cuh:68,
+// enactor_hybrid.cuh:64).
+//
+// Fused searches never write the edge frontier: a level's expansion and the
+// next level's contraction are one pass of the vertex-frontier kernel
+// (ec_kernel), which tests each gathered neighbour instead of storing it for
+// the next pass to read -- 8 bytes per edge and one grid barrier per level less,
+// and for hybrid no hand-off through the host.  R-MAT 22 contract-expand 1060
+// -> 790 us, random 10^6 hybrid 340 -> 167 us.  What the caller sees is kept: labels,
+// search depth, the queue total (the edges of the processed levels) and the
+// overflow of a level larger than the edge frontiers' capacity.  Per-level
+// launches and captured graphs run the two phases as launches of their own
+// (edge_kernel).
 #include "launch_common.cuh"
 
 namespace b40c {
@@ -10,21 +21,17 @@ namespace rt {
 namespace {
 
 template <int B, bool PRED>
-int enact_edge_t(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
-                 int32_t depth_limit)
+int enact_phases_t(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
+                   int32_t depth_limit)
 {
     int rc;
-    const bool pingpong = strategy == B40C_CONTRACT_EXPAND || strategy == B40C_HYBRID;
+    const bool pingpong = strategy != B40C_TWO_PHASE;
     const int64_t ecap = cap_of(p->queue_sizing, p->edges), vcap = cap_of(p->queue_sizing, p->nodes);
     if ((rc = ensure_ef(p, 0, ecap))) return rc;
     if (pingpong && (rc = ensure_ef(p, 1, ecap))) return rc;
     if ((rc = ensure_vf(p, 0, vcap))) return rc;
     if ((rc = ensure_slots(p))) return rc;
     BfsParams k = make_params(p, pol);
-    // hybrid's hand-off: saturation_quit queue items per 256 threads of the grid,
-    // so the frontier size at which it leaves the fused kernel does not move
-    // with the CTA size (the grid of 512-thread CTAs has half as many)
-    k.saturation = (int32_t)std::max<int64_t>(1, (int64_t)pol.saturation_quit * B / 256);
     k.edge_pingpong = pingpong ? 1 : 0;
     k.vcap = (int32_t)p->vcap[0];
     k.ecap = (int32_t)(pingpong ? std::min(p->ecap[0], p->ecap[1]) : p->ecap[0]);
@@ -35,10 +42,9 @@ int enact_edge_t(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int m
     if ((rc = begin_enact(p, src, depth_limit))) return rc;
     if ((rc = begin_instrumented(p))) return rc;
 
-    BfsParams kc = k, kx = k;  // one-phase launches: contract, expand
+    BfsParams kc = k, kx = k;  // contract, expand
     kc.phase_mask = 1;
     kx.phase_mask = 2;
-    kc.max_levels = kx.max_levels = 1;
 
     if (mode == B40C_ENACT_GRAPH) {
         if ((rc = mark_search_start(p))) return rc;
@@ -47,62 +53,15 @@ int enact_edge_t(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int m
         if ((rc = run_graph(p, strategy, init, body, 2))) return rc;
         return finish_timing(p);
     }
+    if (mode != B40C_ENACT_ITERATIVE) return b40c::fail(B40C_ERROR_INVALID_VALUE, "unknown enact mode %d", mode);
     if ((rc = upload_source(p))) return rc;
     if ((rc = launch_init<PRED>(p, k, false, p->needs_init))) return rc;
     if ((rc = mark_search_start(p))) return rc;
-
-    // one level as two launches (contract, expand); returns with the state read back
-    auto two_phase_level = [&]() -> int {
-        int r;
-        if ((r = launch_plain(p, kern, grid, B, smem, kc, "contract launch"))) return r;
-        if ((r = launch_plain(p, kern, grid, B, smem, kx, "expand launch"))) return r;
-        return read_state(p);
-    };
-
-    if (strategy == B40C_HYBRID && mode == B40C_ENACT_FUSED) {
-        BfsParams kf = k;
-        kf.persistent = 1;
-        kf.phase_mask = 3;
-        kf.hybrid = 1;
-        kf.max_levels = INT32_MAX;
-        kf.skip_arrival_cta = injected_skip_cta();
-        kf.late_start_ns = injected_late_start_ns();
-        const int threshold = grid * k.saturation;
-        while (true) {
-            CUDA_TRY(cudaMemsetAsync(&p->st->barrier, 0, sizeof(unsigned long long), p->stream), "barrier reset");
-            CUDA_TRY(cudaMemsetAsync(&p->st->saturated, 0, sizeof(int32_t), p->stream), "flag reset");
-            if ((rc = launch_cooperative(p, kern, grid, B, smem, kf, "cooperative launch of the contract-expand kernel")))
-                return rc;
-            if ((rc = read_state(p))) return rc;
-            if (p->h_st->error || p->h_st->done || !p->h_st->saturated) break;
-            // saturated: two-phase levels until the frontier falls back under the threshold
-            bool finished = false;
-            while (true) {
-                if ((rc = two_phase_level())) return rc;
-                const SearchState &h = *p->h_st;
-                if (h.error || h.done || qe_count(h.qe[(2 * h.cur_level) % 3]) == 0) {
-                    finished = true;
-                    break;
-                }
-                if (qe_count(h.qe[(2 * h.cur_level) % 3]) <= threshold) break;
-            }
-            if (finished) break;
-        }
-    } else if (mode == B40C_ENACT_FUSED) {
-        BfsParams kf = k;
-        kf.persistent = 1;
-        kf.phase_mask = 3;
-        kf.max_levels = INT32_MAX;
-        kf.skip_arrival_cta = injected_skip_cta();
-        kf.late_start_ns = injected_late_start_ns();
-        if ((rc = launch_cooperative(p, kern, grid, B, smem, kf, "cooperative launch of the contract-expand kernel")))
-            return rc;
-    } else if (mode == B40C_ENACT_ITERATIVE) {
+    if ((rc = read_state(p))) return rc;
+    while (!(p->h_st->error || p->h_st->done || qe_count(p->h_st->qe[(2 * p->h_st->cur_level) % 3]) == 0)) {
+        if ((rc = launch_plain(p, kern, grid, B, smem, kc, "contract launch"))) return rc;
+        if ((rc = launch_plain(p, kern, grid, B, smem, kx, "expand launch"))) return rc;
         if ((rc = read_state(p))) return rc;
-        while (!(p->h_st->error || p->h_st->done || qe_count(p->h_st->qe[(2 * p->h_st->cur_level) % 3]) == 0))
-            if ((rc = two_phase_level())) return rc;
-    } else {
-        return b40c::fail(B40C_ERROR_INVALID_VALUE, "unknown enact mode %d", mode);
     }
     return finish_timing(p);
 }
@@ -112,9 +71,19 @@ int enact_edge_t(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int m
 int enact_edge(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
                int32_t depth_limit)
 {
-#define B40C_EDGE(B)                                                                      \
-    (p->mark_pred ? enact_edge_t<B, true>(p, strategy, mode, src, max_grid, pol, depth_limit) \
-                  : enact_edge_t<B, false>(p, strategy, mode, src, max_grid, pol, depth_limit))
+    if (mode == B40C_ENACT_FUSED) {
+        // the capacity the edge frontiers have, or would be given: a larger level
+        // overflows, as it does in the per-phase launches
+        const int64_t ecap = std::max<int64_t>(cap_of(p->queue_sizing, p->edges), 1);
+        const int64_t first = std::max(ecap, p->ecap[0]), second = std::max(ecap, p->ecap[1]);
+        const int64_t limit = strategy == B40C_TWO_PHASE ? first : std::min(first, second);
+        p->queues_edges = true;
+        return enact_vertex(p, mode, src, max_grid, pol, depth_limit, false,
+                            (int32_t)std::min<int64_t>(limit, INT32_MAX - 1));
+    }
+#define B40C_EDGE(B)                                                                                \
+    (p->mark_pred ? enact_phases_t<B, true>(p, strategy, mode, src, max_grid, pol, depth_limit)     \
+                  : enact_phases_t<B, false>(p, strategy, mode, src, max_grid, pol, depth_limit))
     switch (pol.threads) {
     case 128: return B40C_EDGE(128);
     case 512: return B40C_EDGE(512);

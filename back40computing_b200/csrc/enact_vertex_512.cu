@@ -3,6 +3,6 @@
 
 namespace b40c {
 namespace rt {
-template int enact_vertex_b<512>(b40c_bfs_problem *, int, int32_t, int, const b40c_bfs_policy &, int32_t, bool);
+template int enact_vertex_b<512>(b40c_bfs_problem *, int, int32_t, int, const b40c_bfs_policy &, int32_t, bool, int32_t);
 }  // namespace rt
 }  // namespace b40c

@@ -9,17 +9,31 @@ namespace rt {
 
 template <int B, bool PRED>
 int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
-               int32_t depth_limit, bool direction_opt)
+               int32_t depth_limit, bool direction_opt, int32_t edge_limit)
 {
     int rc;
-    if ((rc = ensure_vf(p, 0, cap_of(p->queue_sizing, p->nodes)))) return rc;
-    if ((rc = ensure_vf(p, 1, cap_of(p->queue_sizing, p->nodes)))) return rc;
+    const int64_t vcap = cap_of(p->queue_sizing, p->nodes);
+    VertexFrontier queue[2];
+    int64_t queue_cap = 0;
+    if (edge_limit != INT32_MAX) {
+        if ((rc = edge_strategy_queues(p, vcap, queue, &queue_cap))) return rc;
+    } else {
+        for (int i = 0; i < 2; i++) {
+            if ((rc = ensure_vf(p, i, vcap))) return rc;
+            queue[i] = p->vf[i];
+        }
+        queue_cap = std::min(p->vcap[0], p->vcap[1]);
+    }
     if ((rc = ensure_slots(p))) return rc;
     if (direction_opt && pol.bottom_up_hub_probes > 0 && (rc = ensure_hubs(p))) return rc;
     const bool lists = direction_opt && !PRED && pol.bottom_up_list > 0;
     if (lists && (rc = ensure_unvisited_lists(p))) return rc;
     BfsParams k = make_params(p, pol);
+    k.vf[0] = queue[0];
+    k.vf[1] = queue[1];
+    k.vcap = (int32_t)queue_cap;
     k.direction_opt = direction_opt ? 1 : 0;
+    k.edge_limit = edge_limit;
     if (!direction_opt) k.hub2 = nullptr;
     if (lists) {
         // distance searches: bottom-up levels after the first one scan the unvisited list
@@ -87,10 +101,11 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
 // One CTA size's entry, instantiated in enact_vertex_<B>.cu.
 template <int B>
 int enact_vertex_b(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
-                   int32_t depth_limit, bool direction_optimizing)
+                   int32_t depth_limit, bool direction_optimizing, int32_t edge_limit)
 {
-    return p->mark_pred ? enact_ec_t<B, true>(p, mode, src, max_grid, pol, depth_limit, direction_optimizing)
-                        : enact_ec_t<B, false>(p, mode, src, max_grid, pol, depth_limit, direction_optimizing);
+    return p->mark_pred ? enact_ec_t<B, true>(p, mode, src, max_grid, pol, depth_limit, direction_optimizing, edge_limit)
+                        : enact_ec_t<B, false>(p, mode, src, max_grid, pol, depth_limit, direction_optimizing,
+                                               edge_limit);
 }
 
 }  // namespace rt

@@ -153,7 +153,7 @@ extern "C" int b40c_bfs_search_noalloc(const int32_t *d_row_offsets, const int32
     k.cta_thresh = 512;
     k.warp_cull = 0;
     k.precheck = 1;
-    k.saturation = 512;
+    k.edge_limit = INT32_MAX;
     k.persistent = 1;
     k.skip_arrival_cta = -1;
     k.spin_limit = dev::kSpinLimit;

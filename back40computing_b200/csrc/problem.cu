@@ -76,6 +76,28 @@ int ensure_ef(b40c_bfs_problem *p, int i, int64_t cap)
     return B40C_SUCCESS;
 }
 
+int edge_strategy_queues(b40c_bfs_problem *p, int64_t cap, VertexFrontier (&queue)[2], int64_t *queue_cap)
+{
+    cap = std::max<int64_t>(std::max<int64_t>(cap, 1), p->vcap[0]);
+    const int64_t cf_len = (std::max<int64_t>(p->edges, 1) + dev::kChunkGrain - 1) / dev::kChunkGrain + 2;
+    int next = 0;  // edge frontier not yet taken
+    for (int i = 0; i < 2; i++) {
+        if (p->vcap[i] < cap) {
+            while (next < 2 && p->ecap[next] < 3 * cap + 1 + cf_len) next++;
+            if (next < 2) {
+                int32_t *at = p->ef[next++].v;
+                queue[i] = VertexFrontier{at, at + cap, at + 2 * cap, at + 3 * cap + 1};
+                continue;
+            }
+            const int rc = ensure_vf(p, i, cap);
+            if (rc) return rc;
+        }
+        queue[i] = p->vf[i];
+    }
+    *queue_cap = cap;
+    return B40C_SUCCESS;
+}
+
 int64_t cap_of(double qs, int64_t base)
 {
     double c = std::ceil(qs * (double)base);
@@ -136,7 +158,7 @@ BfsParams make_params(b40c_bfs_problem *p, const b40c_bfs_policy &pol)
     k.cta_thresh = pol.cta_gather_threshold;
     k.warp_cull = pol.warp_cull;
     k.precheck = pol.bitmask_precheck > 0 ? pol.bitmask_precheck : 0;  // -1 (off) must not read as true
-    k.saturation = pol.saturation_quit;
+    k.edge_limit = INT32_MAX;
     k.persistent = 0;
     k.skip_arrival_cta = -1;
     k.spin_limit = test_spin_limit();
@@ -957,6 +979,7 @@ int b40c_bfs_enact_limited(b40c_bfs_problem *p, int strategy, int mode, int32_t 
     default_launch(p, strategy, policy, &pol);
     DeviceGuard guard(p->device);
     p->timed = false;
+    p->queues_edges = false;
     switch (strategy) {
     case B40C_EXPAND_CONTRACT:
         rc = enact_vertex(p, mode, src, max_grid_size, pol, depth_limit, false);
@@ -991,7 +1014,8 @@ int b40c_bfs_stats(b40c_bfs_problem *p, int64_t *total_queued, int32_t *search_d
     int rc = read_state(p);
     if (rc) return rc;
     if ((rc = check_state_errors(p))) return rc;
-    if (total_queued) *total_queued = (int64_t)p->h_st->total_queued;
+    if (total_queued)
+        *total_queued = (int64_t)(p->queues_edges ? p->h_st->visited_edges[p->h_st->cur_level % 3] : p->h_st->total_queued);
     if (search_depth) *search_depth = p->h_st->max_level + 1;
     if (avg_duty) {
         *avg_duty = 0.0;

@@ -93,6 +93,7 @@ struct b40c_bfs_problem {
     int ring_pos = 0, ring_count = 0;
     bool timed = false;
     bool needs_init = true;  // labels/mask dirty since the last reset
+    bool queues_edges = false;  // the last search's queue total is its levels' edges (fused edge strategies)
     // CUDA graphs of whole searches (ENACT_GRAPH), one per strategy, rebuilt
     // when the kernel parameters (buffers, policy) or the grid change
     cudaGraphExec_t graph_exec[5] = {};
@@ -141,6 +142,10 @@ void free_vf(VertexFrontier &f);
 void free_ef(EdgeFrontier &f);
 int ensure_vf(b40c_bfs_problem *p, int i, int64_t cap);
 int ensure_ef(b40c_bfs_problem *p, int i, int64_t cap);
+// The two vertex queues of a fused edge-strategy search, of `cap` entries or as
+// many as the handle's first one has: those it has, else space in the edge
+// frontiers a reset allocated (which the search does not use), else new ones.
+int edge_strategy_queues(b40c_bfs_problem *p, int64_t cap, VertexFrontier (&queue)[2], int64_t *queue_cap);
 int64_t cap_of(double qs, int64_t base);
 int64_t device_bytes(const b40c_bfs_problem *p);
 // A problem handle whose CSR arrays `load` fills (upload, zero-copy mapping or
@@ -174,8 +179,9 @@ struct KernelNode {
 int run_graph(b40c_bfs_problem *p, int slot, const KernelNode &init, KernelNode *body, int n_body);
 
 // enactors
+// `edge_limit`: the largest level accepted, in edges (fused edge-frontier strategies)
 int enact_vertex(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
-                 int32_t depth_limit, bool direction_optimizing);
+                 int32_t depth_limit, bool direction_optimizing, int32_t edge_limit = INT32_MAX);
 int check_symmetric(b40c_bfs_problem *p);
 int ensure_hubs(b40c_bfs_problem *p);
 int ensure_unvisited_lists(b40c_bfs_problem *p);

@@ -87,8 +87,8 @@ typedef struct b40c_bfs_policy {
                                       a multiple of 32 in [256, 2048] (default 2048) */
     int32_t warp_gather_threshold; /* run length at or above which a warp gathers cooperatively (>= 32) */
     int32_t cta_gather_threshold;  /* run length at or above which the CTA gathers with bulk staging */
-    int32_t saturation_quit;       /* hybrid: queue items per CTA of 256 threads (scaled for other CTA sizes)
-                                      above which the search leaves the fused kernel */
+    int32_t saturation_quit;       /* hybrid: accepted (>= 1) and without effect: a fused hybrid search keeps no
+                                      edge frontier, so it never leaves its kernel for per-phase launches */
     int32_t warp_cull;             /* 1: drop duplicate neighbours within a warp before the bitmask test,
                                       -1: do not (default) */
     int32_t bitmask_precheck;      /* 1: read the visited word (through L1) before the atomic test-and-set
