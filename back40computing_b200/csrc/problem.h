@@ -12,6 +12,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <vector>
 
 #include "b40c_bfs.h"
 #include "bfs_state.h"
@@ -69,6 +70,14 @@ struct b40c_bfs_problem {
     unsigned long long *d_duty = nullptr;
     unsigned long long *d_arrive = nullptr;  // [kMaxArrivePasses][kMaxArriveCtas]
     int last_grid = 0;                       // CTAs of the last persistent launch
+    // co-resident CTAs per SM of the kernels this handle has launched, by kernel,
+    // CTA size and dynamic shared memory (persistent_grid)
+    struct Occupancy {
+        const void *kernel;
+        int threads, per_sm;
+        size_t smem;
+    };
+    std::vector<Occupancy> occupancy;
     // frontiers
     b40c::VertexFrontier vf[2] = {};
     int64_t vcap[2] = {0, 0};
@@ -93,6 +102,7 @@ struct b40c_bfs_problem {
     int ring_pos = 0, ring_count = 0;
     bool timed = false;
     bool needs_init = true;  // labels/mask dirty since the last reset
+    bool reset_pending = false;  // a reset's fills may still run on `stream` (b40c_bfs_set_stream waits for them)
     bool queues_edges = false;  // the last search's queue total is its levels' edges (fused edge strategies)
     // CUDA graphs of whole searches (ENACT_GRAPH), one per strategy, rebuilt
     // when the kernel parameters (buffers, policy) or the grid change
