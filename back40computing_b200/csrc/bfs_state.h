@@ -44,6 +44,9 @@ struct alignas(128) SearchState {
     // (-1: none yet) and entries
     int32_t ul_sel[3];
     uint32_t ul_count[3];
+    // batched searches: the sources that reached a vertex in a level, by level % 3
+    // (each CTA adds its own; block 0 turns them into search depths a level on)
+    unsigned long long ms_found[3];
     // ---- line 1: the grid barrier's arrival counter (polled by waiting CTAs)
     alignas(128) unsigned long long barrier;  // arrivals of the current persistent launch
     // ---- line 2: the error word (polled now and then) and launch epilogue counter

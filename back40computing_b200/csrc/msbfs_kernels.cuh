@@ -47,10 +47,10 @@ struct MsSmem {
     unsigned long long fm[kChunkMax + 2];  // frontier mask of run j's vertex
     uint16_t own[kChunkMax];
     int32_t out[kChunkMax];
-    int32_t limits[64];
     int32_t off[64];                 // level_off of each slot
+    int32_t joined;                  // some slot's level_off is not 0
     int32_t jn0, jn1;                // join requests taken at this level end: [jn0, jn1)
-    unsigned long long used;         // slots in use
+    uint32_t error;                  // the error word at the start of the level
     int32_t out_count;
     int32_t flag;
     int32_t q, E;
@@ -59,6 +59,37 @@ struct MsSmem {
     unsigned long long scan_warp[B / 32];
     unsigned long long prefix;
 };
+
+// Labels of the 32 vertices of a warp, source by source, one coalesced store per
+// warp and source: lane's vertex v gets level + 1 (minus the slot's level offset)
+// in the rows of acc's bits.  Dense levels walk all rows with a predicated store
+// each (four instructions a row; finding the next set bit of a 64-bit mask and
+// its row took sixteen, a third of a pull level's instructions): random 2^21
+// batch 1.36 -> 1.23 ms, with the level start below.  All 32 lanes call it.
+template <typename Smem>
+__device__ __forceinline__ void ms_store_labels(const MsParams &m, const Smem &s, int level, long long n, int v,
+                                                unsigned long long acc)
+{
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+        const unsigned bits = half ? (unsigned)(acc >> 32) : (unsigned)acc;
+        unsigned any = __reduce_or_sync(0xffffffffu, bits);
+        int32_t *row = m.labels + (long long)half * 32 * n + v;
+        if (!s.joined && __popc(any) >= 12) {
+#pragma unroll
+            for (int src = 0; src < 32; src++) {
+                if ((bits >> src) & 1u) st_stream(row, level + 1);
+                row += n;
+            }
+        } else {
+            while (any) {
+                const int src = __ffs((int)any) - 1;
+                any &= any - 1;
+                if ((bits >> src) & 1u) st_stream(row + src * n, level + 1 - s.off[half * 32 + src]);
+            }
+        }
+    }
+}
 
 // Push level: expansion of the CTA's share of the level's frontier queue.
 template <int B>
@@ -284,15 +315,7 @@ __device__ __forceinline__ bool ms_pull_block(const BfsParams &p, const MsParams
         fnext[v] = acc;
         s.flag = 1;
     }
-    // labels, source by source: one coalesced store per warp
-    const unsigned long long wor_lo = __reduce_or_sync(0xffffffffu, (unsigned)(acc & 0xffffffffull));
-    const unsigned long long wor_hi = __reduce_or_sync(0xffffffffu, (unsigned)(acc >> 32));
-    unsigned long long wor = wor_lo | (wor_hi << 32);
-    while (wor) {
-        const int src = __ffsll((long long)wor) - 1;
-        wor &= wor - 1;
-        if ((acc >> src) & 1ull) st_stream(m.labels + (long long)src * n + v, level + 1 - s.off[src]);
-    }
+    ms_store_labels(m, s, level, n, v, acc);
     r0_out = r0;
     deg_out = r1 - r0;
     return acc && r1 > r0;
@@ -461,29 +484,43 @@ __global__ void __launch_bounds__(B, 1024 / B) msbfs_kernel(BfsParams p, MsParam
     DutyClock duty(p);
     for (int level = 0;; level++) {
         const int pass = level;
-        // the slots' depth limits and level offsets (sources may have joined at the last level end)
-        if (tid < 64) {
-            s.limits[tid] = ld_cg(m.depth_limit + tid);
-            s.off[tid] = ld_cg(m.level_off + tid);
-        }
-        if (tid == 0) s.used = m.join ? ld_cg64(&m.join->used) : (m.k >= 64 ? ~0ull : ((1ull << m.k) - 1ull));
-        __syncthreads();
-        if (tid == 0) {
+        // warp 0: the slots' depth limits and level offsets (sources may have joined
+        // at the last level end), the counters and the error word, in one round trip
+        if (tid < 32) {
+            const int lim0 = ld_cg(m.depth_limit + tid), lim1 = ld_cg(m.depth_limit + 32 + tid);
+            const int off0 = ld_cg(m.level_off + tid), off1 = ld_cg(m.level_off + 32 + tid);
+            const unsigned long long used =
+                m.join ? ld_cg64(&m.join->used) : (m.k >= 64 ? ~0ull : ((1ull << m.k) - 1ull));
             const unsigned long long x = ld_cg64(&p.st->qe[pass % 3]);
-            s.q = qe_count(x);
-            s.E = qe_edges(x);
-            s.flag = 0;
-            if ((unsigned)s.E > (unsigned)p.edges || (unsigned)s.q > (unsigned)p.vcap) {
-                atomicOr(&p.st->error, kErrOverflow);  // never read a frontier past its arrays
-                s.q = 0;
-            }
-            s.found = 0;
-            unsigned long long act = 0;
-            for (int src = 0; src < 64; src++)
-                if (((s.used >> src) & 1ull) && (s.limits[src] < 0 || level - s.off[src] < s.limits[src]))
-                    act |= 1ull << src;
-            s.active = act;
+            const unsigned error = ld_cg(&p.st->error);
+            // sources that labelled a vertex `level` have search depth level + 1
+            const unsigned long long reached = ld_cg64(&p.st->ms_found[(pass + 2) % 3]);
+            const unsigned act0 = __ballot_sync(0xffffffffu, ((used >> tid) & 1ull) && (lim0 < 0 || level - off0 < lim0));
+            const unsigned act1 =
+                __ballot_sync(0xffffffffu, ((used >> (32 + tid)) & 1ull) && (lim1 < 0 || level - off1 < lim1));
+            const bool joined = __any_sync(0xffffffffu, off0 != 0 || off1 != 0);
+            s.off[tid] = off0;
+            s.off[32 + tid] = off1;
             if (blockIdx.x == 0) {
+                if ((reached >> tid) & 1ull) m.depth[tid] = max(ld_cg(m.depth + tid), level + 1 - off0);
+                if ((reached >> (32 + tid)) & 1ull)
+                    m.depth[32 + tid] = max(ld_cg(m.depth + 32 + tid), level + 1 - off1);
+            }
+            if (tid == 0) {
+                s.q = qe_count(x);
+                s.E = qe_edges(x);
+                s.error = error;
+                s.flag = 0;
+                if ((unsigned)s.E > (unsigned)p.edges || (unsigned)s.q > (unsigned)p.vcap) {
+                    atomicOr(&p.st->error, kErrOverflow);  // never read a frontier past its arrays
+                    s.q = 0;
+                }
+                s.found = 0;
+                s.joined = joined ? 1 : 0;
+                s.active = act0 | ((unsigned long long)act1 << 32);
+            }
+            if (tid == 0 && blockIdx.x == 0) {
+                p.st->ms_found[(pass + 1) % 3] = 0;
                 p.st->qe[(pass + 2) % 3] = 0;
                 p.st->tile_ctr[(pass + 1) % 3] = 0;
                 atomicAdd(&p.st->total_queued, (unsigned long long)s.q);
@@ -499,7 +536,7 @@ __global__ void __launch_bounds__(B, 1024 / B) msbfs_kernel(BfsParams p, MsParam
             }
         }
         __syncthreads();
-        if (s.q == 0 || s.active == 0 || ld_cg(&p.st->error) != 0) break;
+        if (s.q == 0 || s.active == 0 || s.error != 0) break;
         // pull when the frontier's edges are a large share of the graph (symmetric graphs)
         const bool pull = m.pull_ok && (long long)s.E * p.bu_alpha > (long long)p.edges;
         if (tid == 0 && blockIdx.x == 0 && pull && p.levels && pass < kMaxLevelRecords) p.levels[pass].bottom_up = 1;
@@ -518,15 +555,7 @@ __global__ void __launch_bounds__(B, 1024 / B) msbfs_kernel(BfsParams p, MsParam
         }
         __syncthreads();
         if (s.flag) max_level_seen = level + 1;
-        if (tid == 0) {
-            // sources that labelled a vertex level + 1 have search depth >= level + 2
-            unsigned long long bits = s.found;
-            while (bits) {
-                const int src = __ffsll((long long)bits) - 1;
-                bits &= bits - 1;
-                atomicMax(m.depth + src, level + 2 - s.off[src]);
-            }
-        }
+        if (tid == 0 && s.found) atomicOr(&p.st->ms_found[pass % 3], s.found);
         if (!duty.barrier(p.st, generation, &s_ok)) break;
         // clear this level's frontier masks (the queue lists every vertex with edges that has one)
         {
@@ -589,6 +618,7 @@ __global__ void msbfs_init_kernel(BfsParams p, MsParams m)
         st->total_queued = 0;
         st->finished = 0;
         st->qe[1] = st->qe[2] = 0;
+        st->ms_found[0] = st->ms_found[1] = st->ms_found[2] = 0;
     }
 }
 
