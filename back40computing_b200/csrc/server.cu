@@ -194,6 +194,8 @@ const b40c_bfs_policy *batch_policy(const b40c_server *s, const Graph &g, bool s
     *buf = has ? (single ? g.single : g.batch) : b40c_bfs_policy{};
     if (s->ctas_per_sm > 0 && (buf->ctas_per_sm == 0 || buf->ctas_per_sm > s->ctas_per_sm))
         buf->ctas_per_sm = s->ctas_per_sm;
+    // (a share of an SM counts 256-thread CTAs)
+    if (s->ctas_per_sm > 0 && buf->threads == 0) buf->threads = 256;
     return buf;
 }
 
