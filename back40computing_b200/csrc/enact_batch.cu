@@ -34,6 +34,8 @@ void free_batch(b40c_bfs_problem *p)
     p->d_ms_src = nullptr;
     p->d_ms_depth = nullptr;
     p->d_ms_off = nullptr;
+    p->d_ms_seg = nullptr;
+    p->ms_segments = -1;
     p->d_ms_join = p->h_ms_join = nullptr;
     p->ms_seeded_ev = nullptr;
     p->join_stream = nullptr;
@@ -51,7 +53,10 @@ int ensure_batch(b40c_bfs_problem *p, int k)
                 return rc;
         if ((rc = alloc_dev((void **)&p->d_ms_src, sizeof(int32_t) * 64, "batch depth limits"))) return rc;
         if ((rc = alloc_dev((void **)&p->d_ms_depth, sizeof(int32_t) * 64, "batch search depths"))) return rc;
-        if ((rc = alloc_dev((void **)&p->d_ms_off, sizeof(int32_t) * 64, "batch level offsets"))) return rc;
+        if ((rc = alloc_dev((void **)&p->d_ms_off, 512 + sizeof(int2) * max_pull_segments(p->edges),
+                            "batch level offsets")))
+            return rc;
+        p->d_ms_seg = (int2 *)((char *)p->d_ms_off + 512);
         if ((rc = alloc_dev((void **)&p->d_ms_join, sizeof(MsJoin), "batch join requests"))) return rc;
         CUDA_TRY(cudaMallocHost((void **)&p->h_ms_join, sizeof(MsJoin)), "pinned join requests");
         memset(p->h_ms_join, 0, sizeof(MsJoin));
@@ -70,6 +75,24 @@ int ensure_batch(b40c_bfs_problem *p, int k)
     return B40C_SUCCESS;
 }
 
+// Lists the segments of a symmetric problem's longest lists, once: d_ms_seg, in
+// any order, and their number (the word before it).
+int ensure_pull_segments(b40c_bfs_problem *p)
+{
+    if (p->ms_segments >= 0) return B40C_SUCCESS;
+    int32_t *count = p->d_ms_off + 64;
+    int32_t found = 0;
+    CUDA_TRY(cudaMemsetAsync(count, 0, sizeof(int32_t), p->stream), "segment count reset");
+    const int blocks = std::max(1, std::min<int>(p->sms * 8, (int)((p->nodes + 255) / 256)));
+    dev::pull_segments_kernel<<<blocks, 256, 0, p->stream>>>(p->d_ro, (int32_t)p->nodes, p->d_ms_seg,
+                                                             (int32_t)max_pull_segments(p->edges), count);
+    CUDA_TRY(cudaGetLastError(), "segment launch");
+    CUDA_TRY(cudaMemcpyAsync(&found, count, sizeof(int32_t), cudaMemcpyDeviceToHost, p->stream), "segment count read");
+    CUDA_TRY(cudaStreamSynchronize(p->stream), "segment count synchronize");
+    p->ms_segments = (int32_t)std::min<int64_t>(found, max_pull_segments(p->edges));
+    return B40C_SUCCESS;
+}
+
 int enact_batch(b40c_bfs_problem *p, const int32_t *sources, const int32_t *limits, int k, int max_grid,
                 const b40c_bfs_policy &pol)
 {
@@ -80,6 +103,7 @@ int enact_batch(b40c_bfs_problem *p, const int32_t *sources, const int32_t *limi
     if ((rc = ensure_batch(p, k))) return rc;
     if ((rc = check_symmetric(p))) return rc;
     if (p->symmetric == 1 && pol.bottom_up_hub_probes > 0 && (rc = ensure_hubs(p))) return rc;
+    if (p->symmetric == 1 && (rc = ensure_pull_segments(p))) return rc;
     // distinct source vertices with their combined source masks; they travel
     // to the device as kernel arguments, so nothing on the host is reused
     // while an earlier batch is still queued
@@ -112,6 +136,8 @@ int enact_batch(b40c_bfs_problem *p, const int32_t *sources, const int32_t *limi
     m.depth = p->d_ms_depth;
     m.level_off = p->d_ms_off;
     m.join = p->d_ms_join;
+    m.seg = p->d_ms_seg;
+    m.segments = p->symmetric == 1 ? p->ms_segments : 0;
     m.k = k;
     m.rows = p->ms_labels_k;
     m.pull_ok = p->symmetric == 1 ? 1 : 0;
@@ -171,6 +197,13 @@ int b40c_msbfs_enact(b40c_bfs_problem *p, const int32_t *sources, const int32_t 
     // (measured on B200: R-MAT 20 batches 4.46 ms at 1/14, 0.82 ms at 1/6;
     // lattices and uniform graphs unchanged or slightly faster)
     if (!policy || policy->bottom_up_alpha == 0) pol.bottom_up_alpha = kBatchPullAlpha;
+    // the launch where the caller left it open (us per batch of 64): 512 threads --
+    // against 256, random 2^21 1234 / 1186, R-MAT 18 303 / 283 -- and one CTA per SM
+    // up to 2^16 vertices, where the barriers are the cost (random 16,385 61 / 57)
+    if (!policy || policy->threads == 0) {
+        pol.threads = 512;
+        if ((!policy || policy->ctas_per_sm == 0) && p->nodes <= 1 << 16) pol.ctas_per_sm = 1;
+    }
     DeviceGuard guard(p->device);
     return enact_batch(p, sources, depth_limits, k, max_grid_size, pol);
 }

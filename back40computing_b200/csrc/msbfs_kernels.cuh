@@ -37,6 +37,8 @@ struct MsParams {
     int32_t k;
     int32_t rows;                    // label rows allocated (joined slots must be below)
     int32_t pull_ok;                 // 1: the graph is symmetric, dense levels may pull
+    const int2 *seg;                 // (vertex, first edge) of each segment of the lists longer than kPullLongest
+    int32_t segments;
 };
 
 template <int B>
@@ -61,31 +63,31 @@ struct MsSmem {
 };
 
 // Labels of the 32 vertices of a warp, source by source, one coalesced store per
-// warp and source: lane's vertex v gets level + 1 (minus the slot's level offset)
-// in the rows of acc's bits.  Dense levels walk all rows with a predicated store
-// each (four instructions a row; finding the next set bit of a 64-bit mask and
-// its row took sixteen, a third of a pull level's instructions): random 2^21
-// batch 1.36 -> 1.23 ms, with the level start below.  All 32 lanes call it.
-template <typename Smem>
-__device__ __forceinline__ void ms_store_labels(const MsParams &m, const Smem &s, int level, long long n, int v,
-                                                unsigned long long acc)
+// warp and source: lane's vertex v gets `value` (minus the slot's level offset,
+// where `off` is given) in the rows of acc's bits.  Dense masks walk all rows with
+// a predicated store each (four instructions a row; finding the next set bit of
+// a 64-bit mask and its row took sixteen, a third of a pull level's
+// instructions): random 2^21 batch 1.36 -> 1.23 ms, with the level start below.
+// All 32 lanes call it.
+__device__ __forceinline__ void ms_store_rows(int32_t *labels, const int32_t *off, int value, long long n, long long v,
+                                              unsigned long long acc)
 {
 #pragma unroll
     for (int half = 0; half < 2; half++) {
         const unsigned bits = half ? (unsigned)(acc >> 32) : (unsigned)acc;
         unsigned any = __reduce_or_sync(0xffffffffu, bits);
-        int32_t *row = m.labels + (long long)half * 32 * n + v;
-        if (!s.joined && __popc(any) >= 12) {
+        int32_t *row = labels + (long long)half * 32 * n + v;
+        if (!off && __popc(any) >= 12) {
 #pragma unroll
             for (int src = 0; src < 32; src++) {
-                if ((bits >> src) & 1u) st_stream(row, level + 1);
+                if ((bits >> src) & 1u) st_stream(row, value);
                 row += n;
             }
         } else {
             while (any) {
                 const int src = __ffs((int)any) - 1;
                 any &= any - 1;
-                if ((bits >> src) & 1u) st_stream(row + src * n, level + 1 - s.off[half * 32 + src]);
+                if ((bits >> src) & 1u) st_stream(row + src * n, value - (off ? off[half * 32 + src] : 0));
             }
         }
     }
@@ -231,9 +233,106 @@ __device__ __forceinline__ void ms_expand_range(const BfsParams &p, const MsPara
 
 // Pull level (symmetric graphs): one thread per vertex, eight neighbours per
 // step, stopping once every missing source is found; lists longer than
-// kPullLongList are searched by the whole warp afterwards.  Only v's own
-// thread writes V[v] and F[next][v].
+// kPullLongList are searched by the whole warp afterwards, and those longer than
+// kPullLongest in segments spread over the grid (a hub's 50,000 neighbours kept
+// one warp busy for 2.5 of a 3.0 ms R-MAT 20 batch: 0.80 ms).  Only v's own thread writes
+// V[v] and F[next][v], except for the segmented lists.
 constexpr int kPullLongList = 256;
+constexpr int kPullLongest = 2048, kPullSegment = 1024;
+
+// The segments of every list longer than kPullLongest, in any order.
+__global__ void pull_segments_kernel(const int32_t *ro, int32_t nodes, int2 *seg, int32_t cap, int32_t *count)
+{
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nodes; v += gridDim.x * blockDim.x) {
+        const int r0 = ro[v], deg = ro[v + 1] - r0;
+        if (deg <= kPullLongest) continue;
+        const int parts = (deg + kPullSegment - 1) / kPullSegment;
+        const int at = atomicAdd(count, parts);
+        for (int i = 0; i < parts && at + i < cap; i++) seg[at + i] = make_int2(v, r0 + i * kPullSegment);
+    }
+}
+
+// The sources of `missing` that the frontier masks of the neighbours [e, hi)
+// hold, searched by the whole warp, 256 neighbours in flight at a time, until all
+// are found.  All 32 lanes call it and get the result.
+__device__ __forceinline__ unsigned long long ms_pull_list(const BfsParams &p, const unsigned long long *fcur, int e,
+                                                           int hi, unsigned long long missing)
+{
+    const int lane = threadIdx.x & 31;
+    constexpr int U = 8;
+    unsigned long long acc = 0;
+    for (; e < hi; e += 32 * U) {
+        int nb[U];
+#pragma unroll
+        for (int t = 0; t < U; t++) {
+            const int x = e + t * 32 + lane;
+            nb[t] = x < hi ? ld_stream(p.column_indices + x) : -1;
+        }
+        unsigned long long f[U];
+#pragma unroll
+        for (int t = 0; t < U; t++) f[t] = nb[t] >= 0 ? ld_keep64(fcur + nb[t]) : 0ull;
+#pragma unroll
+        for (int t = 0; t < U; t++) acc |= f[t];
+        const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)(acc & missing));
+        const unsigned up = __reduce_or_sync(0xffffffffu, (unsigned)((acc & missing) >> 32));
+        acc = ((unsigned long long)up << 32) | lo;
+        if (acc == missing) break;
+    }
+    return acc;
+}
+
+// The segmented lists of a pull level: each warp of the grid takes segments in
+// turn and claims what it finds for the list's vertex as a push level would --
+// the bits it is first to set are labelled, and the first segment to add to
+// F[next] brings the vertex to the next frontier (warp output bv / bc / bd).
+template <int B>
+__device__ __forceinline__ void ms_pull_segments(const BfsParams &p, const MsParams &m, MsSmem<B> &s, int level,
+                                                 const VertexFrontier &vout, unsigned long long *qe_out,
+                                                 unsigned long long &found, int32_t *bv, int32_t *bc, int32_t *bd,
+                                                 int &count)
+{
+    constexpr int CAP = kChunkMax / (B / 32);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned long long *fcur = m.fmask[level & 1];
+    unsigned long long *fnext = m.fmask[(level + 1) & 1];
+    const long long n = p.nodes;
+    for (int i = warp_slice0(warp); i < m.segments; i += (int)gridDim.x * (B / 32)) {
+        const int2 sg = m.seg[i];
+        const int v = sg.x;
+        const unsigned long long missing = s.active & ~ld_keep64(m.visited + v);
+        if (!missing) continue;  // warp-uniform
+        const int r0 = ld_ro(p.row_offsets + v), r1 = ld_ro(p.row_offsets + v + 1);
+        const unsigned long long acc = ms_pull_list(p, fcur, sg.y, min(sg.y + kPullSegment, r1), missing);
+        if (!acc) continue;
+        unsigned long long set = 0;
+        bool first = false;
+        if (lane == 0) {
+            set = acc & ~atomicOr(m.visited + v, acc);
+            if (set) first = atomicOr(fnext + v, set) == 0ull;
+        }
+        set = __shfl_sync(0xffffffffu, set, 0);
+        if (!set) continue;
+        found |= set;
+        s.flag = 1;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int src = h * 32 + lane;
+            if ((set >> src) & 1ull) st_stream(m.labels + src * n + v, level + 1 - s.off[src]);
+        }
+        if (!__any_sync(0xffffffffu, first)) continue;
+        if (count + 1 > CAP) {
+            warp_emit(p, bv, bc, bd, count, vout, qe_out);
+            __syncwarp();
+            count = 0;
+        }
+        if (lane == 0) {
+            bv[count] = v;
+            bc[count] = r0;
+            bd[count] = r1 - r0;
+        }
+        count++;
+    }
+}
 
 // One warp's block of 32 consecutive vertices [vb, vb + 32) of a pull level,
 // below `re`: every lane takes one vertex, eight neighbours per step, stopping
@@ -275,6 +374,7 @@ __device__ __forceinline__ bool ms_pull_block(const BfsParams &p, const MsParams
         if (h.y >= 0) acc |= ld_keep64(fcur + h.y) & missing;
         if (acc == missing || r1 - r0 <= 2) missing = 0;  // nothing left to look for
     }
+    if (r1 - r0 > kPullLongest) missing = acc = 0;  // ms_pull_segments has it
     const bool longlist = missing && (r1 - r0) > kPullLongList;
     if (missing && !longlist) {
         for (int e = r0; e < r1 && acc != missing;) {
@@ -299,15 +399,8 @@ __device__ __forceinline__ bool ms_pull_block(const BfsParams &p, const MsParams
         const int owner = __ffs(lmask) - 1;
         lmask &= lmask - 1;
         const int lr0 = __shfl_sync(0xffffffffu, r0, owner), lr1 = __shfl_sync(0xffffffffu, r1, owner);
-        const unsigned long long miss = __shfl_sync(0xffffffffu, missing, owner);
-        unsigned long long a = 0;
-        for (int eb = lr0; eb < lr1; eb += 32) {
-            const int ee = eb + lane;
-            if (ee < lr1) a |= ld_keep64(fcur + ld_stream(p.column_indices + ee)) & miss;
-            for (int off = 16; off > 0; off >>= 1) a |= __shfl_xor_sync(0xffffffffu, a, off);
-            if (a == miss) break;
-        }
-        if (lane == owner) acc = a;
+        const unsigned long long a = ms_pull_list(p, fcur, lr0, lr1, __shfl_sync(0xffffffffu, missing, owner));
+        if (lane == owner) acc |= a;
     }
     found |= acc;
     if (acc) {
@@ -315,7 +408,7 @@ __device__ __forceinline__ bool ms_pull_block(const BfsParams &p, const MsParams
         fnext[v] = acc;
         s.flag = 1;
     }
-    ms_store_labels(m, s, level, n, v, acc);
+    ms_store_rows(m.labels, s.joined ? s.off : nullptr, level + 1, n, v, acc);
     r0_out = r0;
     deg_out = r1 - r0;
     return acc && r1 > r0;
@@ -331,6 +424,15 @@ __device__ __forceinline__ void ms_pull_range(const BfsParams &p, const MsParams
 {
     const int tid = threadIdx.x, lane = tid & 31;
     constexpr int PER = kChunkMax / B;
+    if (m.segments > 0) {
+        constexpr int CAP = kChunkMax / (B / 32);
+        const int warp = tid >> 5;
+        int32_t *bv = s.out + warp * CAP, *bc = s.colstart + warp * CAP, *bd = s.rel + warp * CAP;
+        int count = 0;
+        ms_pull_segments<B>(p, m, s, level, vout, qe_out, found, bv, bc, bd, count);
+        if (count) warp_emit(p, bv, bc, bd, count, vout, qe_out);
+        __syncthreads();
+    }
     int rs, re;
     cta_range(p.nodes, blockIdx.x, gridDim.x, rs, re);
     for (int cs = rs; cs < re; cs += kChunkMax) {
@@ -380,6 +482,7 @@ __device__ __forceinline__ void ms_pull_range_warp(const BfsParams &p, const MsP
     int32_t *bc = s.colstart + warp * CAP;
     int32_t *bd = s.rel + warp * CAP;
     int count = 0;  // warp-uniform
+    if (m.segments > 0) ms_pull_segments<B>(p, m, s, level, vout, qe_out, found, bv, bc, bd, count);
     const int n = p.nodes;
     const long long stride = (long long)gridDim.x * NW * 32;
     for (long long b64 = (long long)warp_slice0(warp) * 32; b64 < n; b64 += stride) {
@@ -578,14 +681,7 @@ __global__ void __launch_bounds__(B, 1024 / B) msbfs_kernel(BfsParams p, MsParam
         for (long long vb = ((long long)blockIdx.x * (B / 32) + (tid >> 5)) * 32; vb < n; vb += warps * 32) {
             const long long v = vb + lane;
             const unsigned long long miss = v < n ? ~ld_cg64(m.visited + v) & kmask : 0ull;
-            const unsigned lo = __reduce_or_sync(0xffffffffu, (unsigned)(miss & 0xffffffffull));
-            const unsigned hi = __reduce_or_sync(0xffffffffu, (unsigned)(miss >> 32));
-            unsigned long long wor = ((unsigned long long)hi << 32) | lo;
-            while (wor) {
-                const int src = __ffsll((long long)wor) - 1;
-                wor &= wor - 1;
-                if ((miss >> src) & 1ull) st_stream(m.labels + (long long)src * n + v, -1);
-            }
+            ms_store_rows(m.labels, nullptr, -1, n, v, miss);
         }
     }
     if (tid == 0 && max_level_seen >= 0) atomicMax(&p.st->max_level, max_level_seen);

@@ -322,7 +322,7 @@ int64_t device_bytes(const b40c_bfs_problem *p)
         if (p->vcap[i]) t += 2 * a(4 * p->vcap[i]) + a(4 * (p->vcap[i] + 1)) + a(4 * cf_len);
         if (p->ecap[i]) t += a(4 * p->ecap[i]) * (p->ef[i].pred ? 2 : 1);
     }
-    if (p->d_ms_visited) t += 3 * a(8 * n) + 2 * a(4 * 64);
+    if (p->d_ms_visited) t += 3 * a(8 * n) + 2 * a(4 * 64) + 8 * max_pull_segments(m);
     if (p->d_ms_labels) t += a(4 * n * (int64_t)p->ms_labels_k);
     if (p->d_levels) t += a((int64_t)sizeof(LevelRecord) * kMaxLevelRecords);
     if (p->d_duty) t += a(4 * sizeof(unsigned long long));
@@ -349,7 +349,7 @@ int64_t planned_bytes(int64_t n, int64_t m, int k, double qs)
     t += 2 * (2 * a(4 * cap) + a(4 * (cap + 1)) + a(4 * cf_len));
     t += a(8 * n);      // hub pairs (built by the server for every graph)
     t += 2 * a(4 * n);  // unvisited lists (direction-optimizing distance searches)
-    if (k > 0) t += 3 * a(8 * n) + 2 * a(4 * 64) + a(4 * n * (int64_t)k);
+    if (k > 0) t += 3 * a(8 * n) + 2 * a(4 * 64) + 8 * max_pull_segments(m) + a(4 * n * (int64_t)k);
     return t;
 }
 

@@ -54,7 +54,9 @@ struct b40c_bfs_problem {
     int32_t ms_labels_k = 0;       // sources the label array is sized for
     int32_t *d_ms_src = nullptr;   // [64] depth limit of each source slot
     int32_t *d_ms_depth = nullptr; // [64] search depth of each source slot
-    int32_t *d_ms_off = nullptr;   // [64] level at which each slot's source was seeded
+    int32_t *d_ms_off = nullptr;   // [64] level at which each slot's source was seeded, then
+    int2 *d_ms_seg = nullptr;      // the segments of the lists longer than dev::kPullLongest (in d_ms_off's memory)
+    int32_t ms_segments = -1;      // their number, -1: not built
     int32_t ms_k = 0;              // sources of the last batch
     // sources joining the batch in flight (b40c_msbfs_join): the device request
     // block, its pinned host staging, the stream the requests are copied on and
@@ -197,6 +199,8 @@ int ensure_hubs(b40c_bfs_problem *p);
 int ensure_unvisited_lists(b40c_bfs_problem *p);
 void free_batch(b40c_bfs_problem *p);
 int ensure_batch(b40c_bfs_problem *p, int k);
+// Segments a graph of m edges can have (lists longer than 2048 in parts of 1024).
+inline int64_t max_pull_segments(int64_t m) { return m / 1024 + m / 2048 + 1; }
 // Queues a batched search of k <= 64 sources on p->stream (asynchronous).
 int enact_batch(b40c_bfs_problem *p, const int32_t *sources, const int32_t *limits, int k, int max_grid,
                 const b40c_bfs_policy &pol);

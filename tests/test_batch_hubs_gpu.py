@@ -1,0 +1,56 @@
+"""Batched searches on graphs whose longest lists are searched in segments spread
+over the grid: degrees at the limits (2048 kept whole, 2049 in three segments, an
+exact and a ragged number of segments), hubs reached late, with a joined slot's
+offsets and with CTA-wide pull levels, against the oracle."""
+import numpy as np
+import pytest
+
+import oracle
+from back40computing_b200 import CsrGraph, CsrProblem
+from back40computing_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+DEGREES = (2047, 2048, 2049, 3072, 5000, 9001)
+
+
+def _hubs():
+    """One hub per degree, its leaves shared with the next hub's, a chain of 6
+    before the first hub and a uniform random part that keeps levels dense."""
+    rng = np.random.default_rng(3)
+    leaves = 12000
+    n = 6 + len(DEGREES) + leaves
+    u, v = [np.arange(6)], [np.arange(1, 7)]
+    for i, d in enumerate(DEGREES):
+        u.append(np.full(d, 6 + i))
+        v.append(6 + len(DEGREES) + rng.choice(leaves, d, replace=False))
+    u.append(6 + len(DEGREES) + rng.integers(0, leaves, 30000))
+    v.append(6 + len(DEGREES) + rng.integers(0, leaves, 30000))
+    u, v = np.concatenate(u), np.concatenate(v)
+    g = CsrGraph()
+    g.FromCoo(np.concatenate([u, v]), np.concatenate([v, u]), n)
+    return g
+
+
+@pytest.mark.parametrize("k", [1, 33, 64])
+@pytest.mark.parametrize("knobs", [{}, {"threads": 128}, {"threads": 256, "warp_contract": -1},
+                                   {"threads": 512, "bottom_up_alpha": 1 << 20},
+                                   {"bottom_up_hub_probes": -1, "bottom_up_alpha": 1 << 20}])
+def test_segmented_lists(k, knobs):
+    g = _hubs()
+    p = CsrProblem.from_graph(g)
+    pol = N.Policy()
+    for name, x in knobs.items():
+        setattr(pol, name, x)
+    rng = np.random.default_rng(k)
+    srcs = np.concatenate([[0, 6], rng.integers(0, g.nodes, 62)])[:k].astype(np.int32)
+    limits = np.where(np.arange(k) % 5 == 4, 3, -1).astype(np.int32)
+    p.msbfs(srcs, depth_limits=limits, policy=pol)
+    depths = p.msbfs_depths()
+    for slot in range(k):
+        want, _ = oracle.bfs(g.row_offsets, g.column_indices, int(srcs[slot]))
+        if limits[slot] >= 0:
+            want = np.where(want > limits[slot], -1, want)
+        assert oracle.compare_labels(p.labels_of(slot), want) == -1, f"slot {slot}"
+        assert depths[slot] == int(want.max()) + 1
+    p.Destroy()
