@@ -1964,20 +1964,30 @@ __device__ __forceinline__ unsigned long long ld_cg64(const unsigned long long *
     return v;
 }
 
+// The grid barrier's counter of a persistent launch.  One that sets its search up
+// itself cannot rely on a zero written by an earlier launch's end: two counters
+// take turns, and each launch clears the next one's.
+__device__ __forceinline__ unsigned long long *launch_barrier(const BfsParams &p)
+{
+    return p.init ? &p.st->launch_barrier[p.barrier_sel * 16] : &p.st->barrier;
+}
+
 // Per-CTA busy time (lifetime minus grid-barrier waits), accumulated into
 // p.duty when the search is instrumented: avg duty = busy / lifetime.
 struct DutyClock {
     const BfsParams &p;
     unsigned long long t0 = 0, waited = 0;
-    __device__ explicit DutyClock(const BfsParams &params) : p(params)
+    unsigned long long *counter;  // the launch's grid barrier
+    __device__ DutyClock(const BfsParams &params, unsigned long long *barrier) : p(params), counter(barrier)
     {
         if (p.duty && threadIdx.x == 0) t0 = globaltimer_ns();
     }
     __device__ bool barrier(SearchState *st, unsigned &generation, int *s_flag)
     {
+        // (st: the error word)
         unsigned long long a = 0;
         if (p.duty && threadIdx.x == 0) a = globaltimer_ns();
-        const bool ok = grid_barrier(&st->barrier, generation, &st->error, s_flag, 0, p.spin_limit);
+        const bool ok = grid_barrier(counter, generation, &st->error, s_flag, 0, p.spin_limit);
         if (p.duty && threadIdx.x == 0) waited += globaltimer_ns() - a;
         return ok;
     }
@@ -2106,7 +2116,7 @@ template <int B, bool PRED>
 __device__ __forceinline__ void outside_arrived(const BfsParams &p, ExpandSmem<B, PRED> &s, unsigned generation,
                                                 unsigned outside)
 {
-    if (threadIdx.x == 0) wait_outside_arrivals(&p.st->barrier, generation, outside, &p.st->error, p.spin_limit);
+    if (threadIdx.x == 0) wait_outside_arrivals(launch_barrier(p), generation, outside, &p.st->error, p.spin_limit);
     __syncthreads();
 }
 
@@ -2403,6 +2413,105 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
 // edges are under 1 / kDeferMinShare of the graph's
 constexpr unsigned long long kDeferMinShare = 512;
 
+// Sets up a search: the source's label, visited bit and the level-0
+// frontier, plus the search state.  With FULL it first initialises every
+// label to -1 and the visited mask to 0 (what CsrProblem::Reset does,
+// csr_problem.cuh:723-745), for searches not preceded by a reset and for
+// captured graphs.  The source is read from the state so a captured graph
+// replays with whatever source was uploaded last.
+template <bool PRED, bool VERTEX_FRONTIER, bool FULL>
+__device__ __forceinline__ void init_search(const BfsParams &p)
+{
+    const int src = p.src_by_value ? p.src_arg : p.st->src;
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int src_label = PRED ? -2 : 0;
+    if (FULL) {
+        // 16-byte stores when the labels array is 16-byte aligned (a caller's
+        // array given to the allocation-free search may not be); the source's
+        // label is set by the thread that stores its vector
+        const long long n4 = (reinterpret_cast<uintptr_t>(p.labels) & 15) == 0 ? p.nodes / 4 : 0;
+        int4 *labels4 = reinterpret_cast<int4 *>(p.labels);
+        for (long long i = t0; i < n4; i += stride) {
+            int4 x = make_int4(-1, -1, -1, -1);
+            if (VERTEX_FRONTIER && (src >> 2) == i) {
+                const int r = src & 3;
+                x.x = r == 0 ? src_label : -1;
+                x.y = r == 1 ? src_label : -1;
+                x.z = r == 2 ? src_label : -1;
+                x.w = r == 3 ? src_label : -1;
+            }
+            labels4[i] = x;
+        }
+        for (long long i = 4 * n4 + t0; i < p.nodes; i += stride)
+            p.labels[i] = (VERTEX_FRONTIER && i == src) ? src_label : -1;
+        for (long long w = t0; w < p.mask_words; w += stride) {
+            // edgeless vertices start visited; the source's bit is set for a vertex
+            // frontier and clear for an edge frontier (whose contraction labels it)
+            uint32_t m = p.iso ? p.iso[w] : 0u;
+            if (w == (src >> 5)) m = VERTEX_FRONTIER ? (m | (1u << (src & 31))) : (m & ~(1u << (src & 31)));
+            p.mask[w] = m;
+        }
+    } else if (t0 == 0) {
+        // after a reset (labels -1, mask = the edgeless bits)
+        if (VERTEX_FRONTIER) {
+            p.labels[src] = src_label;
+            p.mask[src >> 5] |= 1u << (src & 31);
+        } else {
+            p.mask[src >> 5] &= ~(1u << (src & 31));
+        }
+    }
+    if (t0 == 0) {
+        SearchState *st = p.st;
+        if (p.src_by_value) {
+            st->src = p.src_arg;
+            st->depth_limit = p.depth_arg;
+        }
+        const int r0 = p.row_offsets[src], r1 = p.row_offsets[src + 1];
+        st->tile_ctr[0] = st->tile_ctr[1] = st->tile_ctr[2] = 0;
+        st->cur_level = 0;
+        st->epoch += 1ull << 24;
+        st->barrier = 0;
+        st->team[0] = st->team[1] = st->team[2] = 0;
+        st->error = 0;
+        st->max_level = 0;
+        st->done = 0;
+        st->total_queued = 0;
+        st->finished = 0;
+        st->qe[1] = st->qe[2] = 0;
+        st->dir[0] = st->dir[1] = st->dir[2] = 0;
+        st->mask_sel[0] = st->mask_sel[1] = st->mask_sel[2] = 0;
+        st->ul_sel[0] = st->ul_sel[1] = st->ul_sel[2] = -1;
+        st->ul_count[0] = st->ul_count[1] = st->ul_count[2] = 0;
+        st->visited_edges[0] = st->visited_edges[1] = st->visited_edges[2] = 0;
+        if (VERTEX_FRONTIER) {
+            const int deg = r1 - r0;
+            st->qe[0] = deg > 0 ? pack(1u, (unsigned)deg) : 0ull;
+            p.vf[0].v[0] = src;
+            p.vf[0].col[0] = r0;
+            p.vf[0].P[0] = 0;
+        } else {
+            // edge frontier: the source is the only item; its predecessor is -2
+            st->qe[0] = pack(1u, 0u);
+            p.ef[0].v[0] = src;
+            if (PRED) p.ef[0].pred[0] = -2;
+        }
+    }
+    if (VERTEX_FRONTIER) {
+        // the source owns every chunk of the level-0 frontier (a hub source has many)
+        const int deg = p.row_offsets[src + 1] - p.row_offsets[src];
+        const long long chunks = min((long long)(deg + kChunkGrain - 1) / kChunkGrain, (long long)p.cf_cap);
+        for (long long c = t0; c < chunks; c += stride) p.vf[0].cf[c] = 0;
+    }
+}
+
+// The set-up as a launch of its own: per-level launches and captured graphs.
+template <bool PRED, bool VERTEX_FRONTIER, bool FULL>
+__global__ void init_kernel(BfsParams p)
+{
+    init_search<PRED, VERTEX_FRONTIER, FULL>(p);
+}
+
 // Expand-contract (vertex frontiers): one level per pass.  With
 // direction_opt, levels with a large frontier run bottom-up.  In a persistent
 // launch, runs of small and mid-size top-down levels are processed by a team of
@@ -2427,12 +2536,23 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
     unsigned bar_phase = 0, generation = 0;
     int max_level_seen = -1;
     late_start(p);
+    if (p.init) {
+        // the search's set-up, by the whole grid, and one barrier (deaf to the error
+        // word, which still holds the last search's until then): a launch of its own
+        // and the gap behind it cost 4 us of a search
+        if (p.init == 2)
+            init_search<PRED, true, true>(p);
+        else
+            init_search<PRED, true, false>(p);
+        if (tid == 0 && blockIdx.x == 0) p.st->launch_barrier[(p.barrier_sel ^ 1) * 16] = 0;
+        if (!grid_barrier(launch_barrier(p), generation, &p.st->error, &s_ok, 0, p.spin_limit, false)) return;
+    }
     int level = ld_cg(&p.st->cur_level);
     bool limit_hit = false, worked = false;
     int phase = 0;          // resident phases so far (the same count in every CTA)
     unsigned team_seq = 0;  // team barriers so far in the search, as of the last phase's end
     const int solo_edges = min(p.small_edges, ExpandSmem<B, PRED>::kEntries);  // largest level of one CTA
-    DutyClock duty(p);
+    DutyClock duty(p, launch_barrier(p));
     __syncthreads();
     for (int iter = 0; iter < p.max_levels; iter++, level++) {
         int pass = level;
@@ -2579,7 +2699,7 @@ __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
     bool limit_hit = false, completed_level = false;
     const int in_idx = p.edge_pingpong ? (level & 1) : 0;
     const int out_idx = p.edge_pingpong ? ((level + 1) & 1) : 0;
-    DutyClock duty(p);
+    DutyClock duty(p, launch_barrier(p));
     __syncthreads();
     if (p.phase_mask & 1) {
         const int pass = 2 * level;
@@ -2621,98 +2741,6 @@ __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
     // the expand launch ends the level; one that broke out (overflow, error) stops
     // the search
     if (p.phase_mask & 2) finish_launch(p, level, 2 * (level + 1), limit_hit, !(completed_level || limit_hit));
-}
-
-// Sets up a search: the source's label, visited bit and the level-0
-// frontier, plus the search state.  With FULL it first initialises every
-// label to -1 and the visited mask to 0 (what CsrProblem::Reset does,
-// csr_problem.cuh:723-745), for searches not preceded by a reset and for
-// captured graphs.  The source is read from the state so a captured graph
-// replays with whatever source was uploaded last.
-template <bool PRED, bool VERTEX_FRONTIER, bool FULL>
-__global__ void init_kernel(BfsParams p)
-{
-    const int src = p.src_by_value ? p.src_arg : p.st->src;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int src_label = PRED ? -2 : 0;
-    if (FULL) {
-        // 16-byte stores when the labels array is 16-byte aligned (a caller's
-        // array given to the allocation-free search may not be); the source's
-        // label is set by the thread that stores its vector
-        const long long n4 = (reinterpret_cast<uintptr_t>(p.labels) & 15) == 0 ? p.nodes / 4 : 0;
-        int4 *labels4 = reinterpret_cast<int4 *>(p.labels);
-        for (long long i = t0; i < n4; i += stride) {
-            int4 x = make_int4(-1, -1, -1, -1);
-            if (VERTEX_FRONTIER && (src >> 2) == i) {
-                const int r = src & 3;
-                x.x = r == 0 ? src_label : -1;
-                x.y = r == 1 ? src_label : -1;
-                x.z = r == 2 ? src_label : -1;
-                x.w = r == 3 ? src_label : -1;
-            }
-            labels4[i] = x;
-        }
-        for (long long i = 4 * n4 + t0; i < p.nodes; i += stride)
-            p.labels[i] = (VERTEX_FRONTIER && i == src) ? src_label : -1;
-        for (long long w = t0; w < p.mask_words; w += stride) {
-            // edgeless vertices start visited; the source's bit is set for a vertex
-            // frontier and clear for an edge frontier (whose contraction labels it)
-            uint32_t m = p.iso ? p.iso[w] : 0u;
-            if (w == (src >> 5)) m = VERTEX_FRONTIER ? (m | (1u << (src & 31))) : (m & ~(1u << (src & 31)));
-            p.mask[w] = m;
-        }
-    } else if (t0 == 0) {
-        // after a reset (labels -1, mask = the edgeless bits)
-        if (VERTEX_FRONTIER) {
-            p.labels[src] = src_label;
-            p.mask[src >> 5] |= 1u << (src & 31);
-        } else {
-            p.mask[src >> 5] &= ~(1u << (src & 31));
-        }
-    }
-    if (t0 == 0) {
-        SearchState *st = p.st;
-        if (p.src_by_value) {
-            st->src = p.src_arg;
-            st->depth_limit = p.depth_arg;
-        }
-        const int r0 = p.row_offsets[src], r1 = p.row_offsets[src + 1];
-        st->tile_ctr[0] = st->tile_ctr[1] = st->tile_ctr[2] = 0;
-        st->cur_level = 0;
-        st->epoch += 1ull << 24;
-        st->barrier = 0;
-        st->team[0] = st->team[1] = st->team[2] = 0;
-        st->error = 0;
-        st->max_level = 0;
-        st->done = 0;
-        st->total_queued = 0;
-        st->finished = 0;
-        st->qe[1] = st->qe[2] = 0;
-        st->dir[0] = st->dir[1] = st->dir[2] = 0;
-        st->mask_sel[0] = st->mask_sel[1] = st->mask_sel[2] = 0;
-        st->ul_sel[0] = st->ul_sel[1] = st->ul_sel[2] = -1;
-        st->ul_count[0] = st->ul_count[1] = st->ul_count[2] = 0;
-        st->visited_edges[0] = st->visited_edges[1] = st->visited_edges[2] = 0;
-        if (VERTEX_FRONTIER) {
-            const int deg = r1 - r0;
-            st->qe[0] = deg > 0 ? pack(1u, (unsigned)deg) : 0ull;
-            p.vf[0].v[0] = src;
-            p.vf[0].col[0] = r0;
-            p.vf[0].P[0] = 0;
-        } else {
-            // edge frontier: the source is the only item; its predecessor is -2
-            st->qe[0] = pack(1u, 0u);
-            p.ef[0].v[0] = src;
-            if (PRED) p.ef[0].pred[0] = -2;
-        }
-    }
-    if (VERTEX_FRONTIER) {
-        // the source owns every chunk of the level-0 frontier (a hub source has many)
-        const int deg = p.row_offsets[src + 1] - p.row_offsets[src];
-        const long long chunks = min((long long)(deg + kChunkGrain - 1) / kChunkGrain, (long long)p.cf_cap);
-        for (long long c = t0; c < chunks; c += stride) p.vf[0].cf[c] = 0;
-    }
 }
 
 }  // namespace dev

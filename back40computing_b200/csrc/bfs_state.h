@@ -49,6 +49,9 @@ struct alignas(128) SearchState {
     unsigned long long ms_found[3];
     // ---- line 1: the grid barrier's arrival counter (polled by waiting CTAs)
     alignas(128) unsigned long long barrier;  // arrivals of the current persistent launch
+    // the same for launches that set their search up themselves: two counters, a line
+    // each, taken in turn
+    alignas(128) unsigned long long launch_barrier[32];
     // ---- line 2: the error word (polled now and then) and launch epilogue counter
     alignas(128) uint32_t error;  // dev::kErr* bits
     uint32_t finished;            // CTAs that finished the current non-persistent launch
@@ -180,6 +183,10 @@ struct BfsParams {
     // depth_arg (and stores them in the state); 0: they were copied into the
     // state before it runs (CUDA-graph replays re-point that copy per launch)
     int32_t src_by_value;
+    // persistent expand-contract launches: 1 the kernel itself sets the search up
+    // after a reset, 2 fills the labels and the mask as well (0: an init launch did)
+    int32_t init;
+    int32_t barrier_sel;  // which launch_barrier this launch uses
     int32_t src_arg, depth_arg;
 };
 

@@ -189,11 +189,11 @@ __device__ __forceinline__ unsigned lanemask_lt()
 // error reported just before the barrier completed is left to the callers'
 // next read of the error word (every caller reads it before its next step, the
 // same value in every CTA), which saves a round trip per barrier.
-// `count` CTAs take part (the whole grid unless given: a sub-grid barrier has
-// its own counter).  `spin_limit` polls bound the wait (kSpinLimit in
+// `count` CTAs take part (the whole grid unless given).  `spin_limit` polls bound the wait (kSpinLimit in
 // production; tests pass a short limit to make a wait run out quickly).
 __device__ __forceinline__ bool grid_barrier(unsigned long long *counter, unsigned &generation, unsigned *error_word,
-                                             int *s_flag, unsigned count = 0, unsigned spin_limit = kSpinLimit)
+                                             int *s_flag, unsigned count = 0, unsigned spin_limit = kSpinLimit,
+                                             bool heed_error = true)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -208,7 +208,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned long long *counter, unsign
                 ok = 0;
                 break;
             }
-            if ((spins & 15) == 0 && ld_cg(error_word) != 0) {
+            if ((spins & 15) == 0 && heed_error && ld_cg(error_word) != 0) {
                 ok = 0;
                 break;
             }

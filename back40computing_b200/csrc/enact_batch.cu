@@ -150,6 +150,8 @@ int enact_batch(b40c_bfs_problem *p, const int32_t *sources, const int32_t *limi
                                        : sizeof(dev::MsSmem<256>);
     int grid = 0;
     if ((rc = persistent_grid(p, kern, pol, max_grid, smem, &grid))) return rc;
+    p->enact_events[0] = p->ev0;
+    p->enact_events[1] = p->ev1;
     CUDA_TRY(cudaEventRecord(p->ev0, p->stream), "event record");
     if ((rc = begin_instrumented(p))) return rc;
     // join requests still being copied for an earlier batch land before this

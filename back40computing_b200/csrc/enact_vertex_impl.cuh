@@ -57,7 +57,7 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
     const size_t smem = kernel_smem<dev::ExpandSmem<B, PRED>>(pol);
     int grid = 0;
     if ((rc = persistent_grid(p, kern, pol, max_grid, smem, &grid))) return rc;
-    if ((rc = begin_enact(p, src, depth_limit))) return rc;
+    if ((rc = begin_enact(p, src, depth_limit, mode == B40C_ENACT_FUSED))) return rc;
     if ((rc = begin_instrumented(p))) return rc;
     if (mode == B40C_ENACT_GRAPH) {
         if ((rc = mark_search_start(p))) return rc;
@@ -72,16 +72,27 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
     k.src_by_value = 1;
     k.src_arg = src;
     k.depth_arg = depth_limit;
-    if ((rc = launch_init<PRED>(p, k, true, p->needs_init))) return rc;
-    if ((rc = mark_search_start(p))) return rc;
     if (mode == B40C_ENACT_FUSED) {
+        // the kernel sets the search up itself: one launch less (see ec_kernel).  A
+        // launch captured into a graph may be replayed, but its turn of the barrier
+        // counters may not: it keeps the set-up launch, which clears the one it uses
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        CUDA_TRY(cudaStreamIsCapturing(p->stream, &capture), "capture query");
+        const bool captured = capture != cudaStreamCaptureStatusNone;
+        if (captured && (rc = launch_init<PRED>(p, k, true, p->needs_init))) return rc;
+        if ((rc = mark_search_start(p))) return rc;
+        k.init = captured ? 0 : p->needs_init ? 2 : 1;
+        k.barrier_sel = p->barrier_sel;
         k.persistent = 1;
         k.max_levels = INT32_MAX;
         k.skip_arrival_cta = injected_skip_cta();
         k.late_start_ns = injected_late_start_ns();
         if ((rc = launch_cooperative(p, kern, grid, B, smem, k, "cooperative launch of the expand-contract kernel")))
             return rc;
+        if (!captured) p->barrier_sel ^= 1;  // (this launch clears the other counter)
     } else if (mode == B40C_ENACT_ITERATIVE) {
+        if ((rc = launch_init<PRED>(p, k, true, p->needs_init))) return rc;
+        if ((rc = mark_search_start(p))) return rc;
         // one launch per level; the host reads the next frontier's size
         for (int level = 0;; level++) {
             if ((rc = read_state(p))) return rc;

@@ -46,17 +46,21 @@ int launch_init(b40c_bfs_problem *p, const BfsParams &k, bool vertex_frontier, b
 }
 
 // Common start of an enact: stores (source, depth limit) in this enact's
-// pinned ring slot and records the enact's start event.  The slot was last
+// pinned ring slot and records the enact's start event (unless the search's own
+// pair of ring events brackets the whole enact, `one_launch`: each event between two
+// searches' kernels costs the stream about a microsecond).  The slot was last
 // used kRing enacts ago; its search (and so its upload) must have finished
 // before the pair is overwritten.
-inline int begin_enact(b40c_bfs_problem *p, int32_t src, int32_t depth_limit)
+inline int begin_enact(b40c_bfs_problem *p, int32_t src, int32_t depth_limit, bool one_launch = false)
 {
     const int slot = p->ring_pos;
     if (p->ring_count == b40c_bfs_problem::kRing)
         CUDA_TRY(cudaEventSynchronize(p->ring_b[slot]), "source slot reuse wait");
     p->h_src_ring[2 * slot] = src;
     p->h_src_ring[2 * slot + 1] = depth_limit;
-    CUDA_TRY(cudaEventRecord(p->ev0, p->stream), "event record");
+    p->enact_events[0] = one_launch ? p->ring_a[slot] : p->ev0;
+    p->enact_events[1] = one_launch ? p->ring_b[slot] : p->ev1;
+    if (!one_launch) CUDA_TRY(cudaEventRecord(p->ev0, p->stream), "event record");
     return B40C_SUCCESS;
 }
 

@@ -584,7 +584,7 @@ __global__ void __launch_bounds__(B, 1024 / B) msbfs_kernel(BfsParams p, MsParam
     const int tid = threadIdx.x;
     unsigned generation = 0;
     int max_level_seen = -1;
-    DutyClock duty(p);
+    DutyClock duty(p, &p.st->barrier);
     for (int level = 0;; level++) {
         const int pass = level;
         // warp 0: the slots' depth limits and level offsets (sources may have joined

@@ -417,7 +417,7 @@ int persistent_grid(b40c_bfs_problem *p, const void *kernel, const b40c_bfs_poli
 int finish_timing(b40c_bfs_problem *p)
 {
     CUDA_TRY(cudaEventRecord(p->ring_b[p->ring_pos], p->stream), "event record");
-    CUDA_TRY(cudaEventRecord(p->ev1, p->stream), "event record");
+    if (p->enact_events[1] == p->ev1) CUDA_TRY(cudaEventRecord(p->ev1, p->stream), "event record");
     p->ring_pos = (p->ring_pos + 1) % b40c_bfs_problem::kRing;
     p->ring_count = std::min(p->ring_count + 1, b40c_bfs_problem::kRing);
     p->timed = true;
@@ -1134,8 +1134,8 @@ int b40c_bfs_last_elapsed_ms(b40c_bfs_problem *p, float *ms)
     if (!p || !ms) return b40c::fail(B40C_ERROR_INVALID_VALUE, "null argument");
     if (!p->timed) return b40c::fail(B40C_ERROR_NOT_READY, "no timed search");
     DeviceGuard guard(p->device);
-    CUDA_TRY(cudaEventSynchronize(p->ev1), "event synchronize");
-    CUDA_TRY(cudaEventElapsedTime(ms, p->ev0, p->ev1), "event elapsed");
+    CUDA_TRY(cudaEventSynchronize(p->enact_events[1]), "event synchronize");
+    CUDA_TRY(cudaEventElapsedTime(ms, p->enact_events[0], p->enact_events[1]), "event elapsed");
     return B40C_SUCCESS;
 }
 

@@ -97,6 +97,7 @@ struct b40c_bfs_problem {
     // streams / timing
     cudaStream_t stream = nullptr, own_stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t enact_events[2] = {nullptr, nullptr};  // around the last enact: ev0 / ev1, or its ring pair
     // ring of event pairs bracketing the search kernels (after source set-up)
     // of the most recent enacts, for per-launch device times
     static constexpr int kRing = 256;
@@ -104,6 +105,7 @@ struct b40c_bfs_problem {
     int ring_pos = 0, ring_count = 0;
     bool timed = false;
     bool needs_init = true;  // labels/mask dirty since the last reset
+    int barrier_sel = 0;     // launch barrier of the next persistent search
     bool reset_pending = false;  // a reset's fills may still run on `stream` (b40c_bfs_set_stream waits for them)
     bool queues_edges = false;  // the last search's queue total is its levels' edges (fused edge strategies)
     // CUDA graphs of whole searches (ENACT_GRAPH), one per strategy, rebuilt

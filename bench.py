@@ -817,7 +817,7 @@ def main():
                          "bytes_per_search_alg": float(balg.mean()),
                          "kernel_ms_per_search": float(kernel_ms.mean())},
             "cpu_baseline": cpu, "e2e": e2e, "topdown": topdown,
-            "gpu_launches": 2 * len(srcs) * args.steps,
+            "gpu_launches": (1 if args.mode == 0 else 2) * len(srcs) * args.steps,
             "clocks": clk,
             **extras,
             "edges_per_search": float(ec.mean()), "search_gteps_mean": float((ec / 1e9).mean()

@@ -300,8 +300,9 @@ int b40c_bfs_level_records(b40c_bfs_problem *problem, b40c_level_record *out, in
 int b40c_bfs_last_elapsed_ms(b40c_bfs_problem *problem, float *ms);
 
 /* Device times (ms) of the search kernels of the last `count` enacts (oldest
- * first; at most 256 are kept): each spans from after the source set-up to
- * the end of the last level, per launch mode.  Synchronises on the newest. */
+ * first; at most 256 are kept): each spans from after the source set-up launch to
+ * the end of the last level, per launch mode (a fused search's kernel does its own
+ * set-up, which is in its time).  Synchronises on the newest. */
 int b40c_bfs_recent_search_ms(b40c_bfs_problem *problem, int count, float *out);
 
 /* GraphSlice device pointers (csr_problem.cuh:99-173). */
