@@ -405,7 +405,11 @@ int coo_to_csr_device(const int32_t *d_rows, const int32_t *d_cols, int64_t node
     // kernels clear and scan the counters of 32 digits at a time)
     int row_bits = 1;
     while (row_bits < 31 && ((int64_t)1 << row_bits) < nodes) row_bits++;
-    const int passes = (row_bits + kMaxDigitBits - 1) / kMaxDigitBits;
+    // (a single pass would write columns over input it has not read, where a caller
+    // converts in place)
+    const auto overlaps = [&](const int32_t *in) { return in < d_ci + edges && d_ci < in + edges; };
+    const int fewest = (row_bits + kMaxDigitBits - 1) / kMaxDigitBits;
+    const int passes = fewest == 1 && (overlaps(d_rows) || overlaps(d_cols)) ? 2 : fewest;
     const int bits = std::max(5, (row_bits + passes - 1) / passes);
     const int ctas = sms * kCtasPerSm;
 

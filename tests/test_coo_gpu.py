@@ -64,6 +64,23 @@ def test_radix_pass_edges(n, m, kind):
     assert np.array_equal(ci, want_ci)
 
 
+@pytest.mark.parametrize("n", [200, 1500, 70000])
+def test_columns_converted_in_place(n):
+    """The column array may take the result: every pass but the last writes elsewhere."""
+    import torch
+    rng = np.random.default_rng(n)
+    rows, cols = rng.integers(0, n, 100001), rng.integers(0, n, 100001)
+    d_r = torch.from_numpy(rows.astype(np.int32)).cuda()
+    d_c = torch.from_numpy(cols.astype(np.int32)).cuda()
+    d_ro = torch.empty(n + 1, dtype=torch.int32, device="cuda")
+    assert N.lib().b40c_coo_to_csr_device(C.c_void_p(d_r.data_ptr()), C.c_void_p(d_c.data_ptr()), n, rows.size,
+                                          C.c_void_p(d_ro.data_ptr()), C.c_void_p(d_c.data_ptr()),
+                                          C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    want_ro, want_ci = _host_csr(n, rows, cols)
+    assert np.array_equal(d_ro.cpu().numpy(), want_ro)
+    assert np.array_equal(d_c.cpu().numpy(), want_ci)
+
+
 def test_rejects_ids_out_of_range():
     rows = np.array([0, 1, 5], np.int32)
     cols = np.array([1, 2, 0], np.int32)
