@@ -239,8 +239,8 @@ __device__ __forceinline__ bool warp_cull(bool valid, int v)
     return valid && (__ffs(peers) - 1 == lane);
 }
 
-// Passes of fewer items than this test without the pre-check: they have few
-// duplicates, and its round trip costs more than the atomics it saves.
+// Passes of fewer items than this, and than vertices, test without the pre-check:
+// they have few duplicates, and its round trip costs more than the atomics it saves.
 constexpr int kPrecheckItems = 1 << 16;
 
 // Discovery of up to U gathered neighbours per thread, in overlapped phases
@@ -261,7 +261,11 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
 {
     bool go[U];
     unsigned word[U];
-    const bool precheck = p.precheck && items >= kPrecheckItems && !(LISTS && s.ul_in >= 0);
+    // more items than vertices: most lose, and all meet on few mask and row lines, so
+    // only winners read their rows (random 2154 x 16, a level of 43 thousand edges
+    // launched by itself: 15.1 -> 5.5 us)
+    const bool busy = items > p.nodes;
+    const bool precheck = p.precheck && (items >= kPrecheckItems || busy) && !(LISTS && s.ul_in >= 0);
     uint32_t *hist = s.hist;
 #pragma unroll
     for (int t = 0; t < U; t++) {
@@ -306,13 +310,19 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
 #pragma unroll
         for (int t = 0; t < U; t++) {
             r0[t] = r1[t] = 0;
-            if (go[t]) {
+            if (go[t] && !busy) {
                 r0[t] = ld_ro(p.row_offsets + v[t]);
                 r1[t] = ld_ro(p.row_offsets + v[t] + 1);
             }
         }
 #pragma unroll
-        for (int t = 0; t < U; t++) found[t] = !((old[t] >> (v[t] & 31)) & 1u);
+        for (int t = 0; t < U; t++) {
+            found[t] = !((old[t] >> (v[t] & 31)) & 1u);
+            if (found[t] && busy) {
+                r0[t] = ld_ro(p.row_offsets + v[t]);
+                r1[t] = ld_ro(p.row_offsets + v[t] + 1);
+            }
+        }
     }
 #pragma unroll
     for (int t = 0; t < U; t++)
@@ -2247,9 +2257,10 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
     __syncthreads();
     unsigned long long tot = 0;
     // a level of more edges than the graph has vertices meets visited ones mostly,
-    // and on few mask words: its atomics alone would queue up (random 20,000
-    // vertices, 237 thousand edges: 33 us, with the pre-check 10)
-    bool precheck = p.precheck && s.E > p.nodes;
+    // and on few mask and row lines, where requests queue up: it tests with the
+    // pre-check (through L1), and only winners read their rows (random 20,000 x 8,
+    // 237 thousand edges, 256-thread CTAs: 24.4 -> 11.8 us)
+    bool busy = s.E > p.nodes;
     for (int run = 0;; run++) {
         if (E > 0) stamp(p, level, 0);
         fill_owners<B>(s, n);
@@ -2280,10 +2291,10 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
                 }
             }
         } else {
-            if (precheck) {
+            if (busy && p.precheck) {
                 unsigned word[PER];
 #pragma unroll
-                for (int t = 0; t < PER; t++) word[t] = v[t] >= 0 ? ld_cg(s.mask + (v[t] >> 5)) : 0u;
+                for (int t = 0; t < PER; t++) word[t] = v[t] >= 0 ? ld_mask(s.mask + (v[t] >> 5)) : 0u;
 #pragma unroll
                 for (int t = 0; t < PER; t++)
                     if ((word[t] >> (v[t] & 31)) & 1u) v[t] = -1;
@@ -2297,14 +2308,20 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
 #pragma unroll
             for (int t = 0; t < PER; t++) {
                 r0[t] = deg[t] = 0;
-                if (v[t] >= 0) {
+                if (v[t] >= 0 && !busy) {
                     r0[t] = ld_ro(p.row_offsets + v[t]);
                     deg[t] = ld_ro(p.row_offsets + v[t] + 1);
                 }
             }
 #pragma unroll
             for (int t = 0; t < PER; t++)
-                if (!((old[t] >> (v[t] & 31)) & 1u)) found |= 1u << t;
+                if (!((old[t] >> (v[t] & 31)) & 1u)) {
+                    found |= 1u << t;
+                    if (busy) {
+                        r0[t] = ld_ro(p.row_offsets + v[t]);
+                        deg[t] = ld_ro(p.row_offsets + v[t] + 1);
+                    }
+                }
         }
         unsigned cnt = 0;
         unsigned long long sum = 0;
@@ -2358,7 +2375,7 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
             (BU && team > 1 &&
              choose_bottom_up(p, false, n_all, E_all, visited + (unsigned long long)(unsigned)E_all)))
             break;
-        precheck = p.precheck && E_all > p.nodes;
+        busy = E_all > p.nodes;
         visited += (unsigned long long)(unsigned)E_all;
         queued += (unsigned long long)(unsigned)n_all;
         if (run == 0 && blockIdx.x == 0) {

@@ -90,3 +90,27 @@ def test_team_levels(kind, threads, knobs, preds):
             if limit < 0:
                 assert queued == int((want >= 0).sum()) - 1
     p.Destroy()
+
+
+@pytest.mark.parametrize("n,degree", [(2, 40), (33, 200), (2154, 16), (20000, 8)])
+@pytest.mark.parametrize("threads,precheck", [(0, 0), (256, 0), (256, -1), (512, 0)])
+def test_levels_of_more_edges_than_vertices(n, degree, threads, precheck):
+    """Few vertices, many edges: team levels and levels launched one by one."""
+    rng = np.random.default_rng(n)
+    u, v = rng.integers(0, n, n * degree), rng.integers(0, n, n * degree)
+    g = _undirected(n, [u], [v])
+    want, _ = oracle.bfs(g.row_offsets, g.column_indices, 0)
+    pol = None
+    if threads:
+        pol = N.Policy()
+        pol.threads, pol.bitmask_precheck = threads, precheck
+    for preds in (False, True):
+        p = CsrProblem.from_graph(g, mark_predecessors=preds)
+        for mode in (N.ENACT_FUSED, N.ENACT_ITERATIVE, N.ENACT_GRAPH):
+            got = search(p, 0, strategy=EXPAND_CONTRACT, policy=pol, mode=mode)
+            assert np.array_equal(got != -1, want != -1)
+            if preds:
+                reached = np.flatnonzero(got >= 0)
+                assert np.array_equal(want[got[reached]] + 1, want[reached])
+            else:
+                assert oracle.compare_labels(got, want) == -1
