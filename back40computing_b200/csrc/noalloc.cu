@@ -22,6 +22,13 @@ namespace noalloc {
 constexpr int64_t kMaxNodes = 1 << 18;  // 262,144 vertices
 constexpr int64_t kMaxEdges = 1 << 22;  // 4,194,304 directed edges
 constexpr int kThreads = 256;
+// Graphs of up to this many edges run one 512-thread CTA per SM (default_launch's
+// rule; us per call against four of 256: random 20,000 x 8 126 / 94, 80,707 x 2
+// 134 / 119), larger ones four of 256, their large levels warp by warp.  Neither
+// asks for shared memory past the kernel's own arrays, so no other search of the
+// same kernel can leave its limit too low for these launches.
+constexpr int64_t kSmallEdges = 1 << 21;
+constexpr int kSmallThreads = 512;
 
 // Byte layout of the scratch array (every piece 256-byte aligned).
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -47,6 +54,7 @@ __global__ void seed_kernel(SearchState *st, int32_t src)
 struct DeviceSetup {
     unsigned char *scratch = nullptr;  // device address of g_scratch on this device
     int grid = 0;                      // co-resident CTAs of the expand-contract kernel
+    int small_grid = 0;                // one per SM, for graphs of up to kSmallEdges
     int init_grid = 0;
 };
 
@@ -70,17 +78,24 @@ static int set_up(int device, DeviceSetup **out)
             return b40c::fail((int)e, "cudaGetSymbolAddress of the search scratch failed: %s", cudaGetErrorString(e));
         }
         const void *kern = (const void *)dev::ec_kernel<kThreads, false, false, false>;
+        const void *small = (const void *)dev::ec_kernel<kSmallThreads, false, false, false>;
         const size_t smem = sizeof(dev::ExpandSmem<kThreads, false>);
+        const size_t small_smem = sizeof(dev::ExpandSmem<kSmallThreads, false>);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        int per_sm = 0, sms = 0;
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem);
+        int per_sm = 0, small_per_sm = 0, sms = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small_per_sm, small, kSmallThreads, small_smem);
         if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (e != cudaSuccess || per_sm < 1) {
+        if (e != cudaSuccess || per_sm < 1 || small_per_sm < 1) {
             cudaGetLastError();
             return b40c::fail(e != cudaSuccess ? (int)e : B40C_ERROR_INVALID_CONFIGURATION,
                               "no-allocation search set-up failed: %s", cudaGetErrorString(e));
         }
         d.grid = per_sm * sms;
+        d.small_grid = sms;
         d.init_grid = sms * 8;
         d.scratch = (unsigned char *)ptr;
     }
@@ -159,6 +174,7 @@ extern "C" int b40c_bfs_search_noalloc(const int32_t *d_row_offsets, const int32
     k.spin_limit = dev::kSpinLimit;
     k.bulk_ok = 1;  // device memory; the kernel aligns each bulk copy by address
     k.alloc_lookback = 0;  // one packed atomic per tile: no look-back slots needed
+    k.warp_contract = edges > kSmallEdges ? 1 : 0;
     k.direction_opt = 0;
     k.bu_alpha = 14;
     k.bu_beta = 24;
@@ -181,8 +197,13 @@ extern "C" int b40c_bfs_search_noalloc(const int32_t *d_row_offsets, const int32
     }
     if (e == cudaSuccess) {
         void *args[] = {&k};
-        e = cudaLaunchCooperativeKernel((const void *)dev::ec_kernel<kThreads, false, false, false>, dim3(d->grid), dim3(kThreads),
-                                        args, sizeof(dev::ExpandSmem<kThreads, false>), stream);
+        if (edges <= kSmallEdges)
+            e = cudaLaunchCooperativeKernel((const void *)dev::ec_kernel<kSmallThreads, false, false, false>,
+                                            dim3(d->small_grid), dim3(kSmallThreads), args,
+                                            sizeof(dev::ExpandSmem<kSmallThreads, false>), stream);
+        else
+            e = cudaLaunchCooperativeKernel((const void *)dev::ec_kernel<kThreads, false, false, false>, dim3(d->grid),
+                                            dim3(kThreads), args, sizeof(dev::ExpandSmem<kThreads, false>), stream);
     }
     // wait for the search and read its error word into a local variable
     unsigned error_word = 0;
