@@ -280,14 +280,17 @@ int resolve_policy(int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *out
 // or 0 in it), each where it measured fastest (us per search):
 //  * 512 threads: against 256, R-MAT 22 direction-optimizing 135 / 119, R-MAT 20
 //    expand-contract 277 / 235 and its predecessors 330 / 272, R-MAT 16 73 / 63,
-//    grid3d-201 3900 / 3540 (list mode and a sub-grid threshold need 256);
+//    grid3d-201 3900 / 3540 (list mode and a sub-grid threshold need 256, and
+//    CTA-wide sub-rounds, warp_contract -1, want four CTAs' in flight: R-MAT 22
+//    expand-contract 1840 / 2540);
 //  * one CTA per SM while the graph is small, where a level's cost is its barriers:
 //    direction-optimizing searches up to 2^19 vertices (R-MAT 16 63 / 55, R-MAT
 //    19 69 / 64, but random 10^6 112 / 130), top-down ones up to 2^21 edges
 //    (R-MAT 13 and random 20,000 107 / 67 and 100 / 62, R-MAT 17 88 / 92).
 void default_launch(const b40c_bfs_problem *p, int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *pol)
 {
-    if ((!in || in->threads == 0) && pol->bottom_up_list <= 0 && pol->subgrid_frontier_edges <= 0) {
+    if ((!in || in->threads == 0) && pol->bottom_up_list <= 0 && pol->subgrid_frontier_edges <= 0 &&
+        pol->warp_contract > 0) {
         pol->threads = 512;
         // as resolve_policy gives the prefetch for a caller's 512
         if (!in || in->bottom_up_prefetch == 0) pol->bottom_up_prefetch = pol->warp_bottom_up < 0 ? 1 : -1;
