@@ -299,7 +299,11 @@ __device__ __forceinline__ void ms_pull_segments(const BfsParams &p, const MsPar
     for (int i = warp_slice0(warp); i < m.segments; i += (int)gridDim.x * (B / 32)) {
         const int2 sg = m.seg[i];
         const int v = sg.x;
-        const unsigned long long missing = s.active & ~ld_keep64(m.visited + v);
+        // other warps set bits of this word meanwhile, and the warp's way through its
+        // collectives follows from it: one lane reads it for all
+        unsigned long long missing = 0;
+        if (lane == 0) missing = s.active & ~ld_keep64(m.visited + v);
+        missing = __shfl_sync(0xffffffffu, missing, 0);
         if (!missing) continue;  // warp-uniform
         const int r0 = ld_ro(p.row_offsets + v), r1 = ld_ro(p.row_offsets + v + 1);
         const unsigned long long acc = ms_pull_list(p, fcur, sg.y, min(sg.y + kPullSegment, r1), missing);

@@ -54,3 +54,26 @@ def test_segmented_lists(k, knobs):
         assert oracle.compare_labels(p.labels_of(slot), want) == -1, f"slot {slot}"
         assert depths[slot] == int(want.max()) + 1
     p.Destroy()
+
+
+@pytest.mark.parametrize("warp_contract", [1, -1])
+def test_many_warps_claim_one_hub(warp_contract):
+    """A hub in 196 segments, first reached by 64 sources at once: the segments'
+    warps read and set the hub's word while the others do."""
+    leaves = 200_000
+    hub = np.zeros(leaves, np.int64)
+    leaf = np.arange(1, leaves + 1)
+    g = CsrGraph()
+    g.FromCoo(np.concatenate([hub, leaf]), np.concatenate([leaf, hub]), leaves + 1)
+    p = CsrProblem.from_graph(g)
+    pol = N.Policy()
+    pol.bottom_up_alpha, pol.warp_contract, pol.bottom_up_hub_probes = 1 << 20, warp_contract, -1
+    for run in range(20):
+        srcs = np.random.default_rng(run).choice(leaf, 64, replace=False).astype(np.int32)
+        p.msbfs(srcs, policy=pol)
+        assert (p.msbfs_depths() == 3).all()
+        for slot in (0, 31, 63):
+            want = np.full(leaves + 1, 2, np.int32)
+            want[[0, srcs[slot]]] = 1, 0
+            assert np.array_equal(p.labels_of(slot), want)
+    p.Destroy()
