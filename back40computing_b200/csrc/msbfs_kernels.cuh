@@ -464,7 +464,9 @@ __device__ __forceinline__ void ms_pull_range(const BfsParams &p, const MsParams
             }
         }
         __syncthreads();
-        emit_frontier<B>(p, s, level, vout, qe_out);
+        // (look-back slots start at 0: not beside the segments' flushes, which take
+        // theirs from the pass counter)
+        emit_frontier<B>(p, s, level, vout, qe_out, m.segments == 0);
         __syncthreads();
     }
 }
@@ -570,7 +572,9 @@ __device__ __forceinline__ void take_joins(const BfsParams &p, const MsParams &m
         }
     }
     __syncthreads();
-    emit_frontier<B>(p, s, level, vout, qe_out);
+    // (from the pass counter, which every way of taking slots leaves at the level's
+    // total: the level may have been flushed warp by warp)
+    emit_frontier<B>(p, s, level, vout, qe_out, false);
     __syncthreads();
     if (tid == 0) {
         __threadfence();
