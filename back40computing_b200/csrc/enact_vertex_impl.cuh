@@ -75,11 +75,12 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
     if (mode == B40C_ENACT_FUSED) {
         // the kernel sets the search up itself: one launch less (see ec_kernel).  A
         // launch captured into a graph may be replayed, but its turn of the barrier
-        // counters may not: it keeps the set-up launch, which clears the one it uses
+        // counters may not: it keeps the set-up launch, which clears the one it uses,
+        // and fills the labels and the mask, which a replay finds as any search left them
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         CUDA_TRY(cudaStreamIsCapturing(p->stream, &capture), "capture query");
         const bool captured = capture != cudaStreamCaptureStatusNone;
-        if (captured && (rc = launch_init<PRED>(p, k, true, p->needs_init))) return rc;
+        if (captured && (rc = launch_init<PRED>(p, k, true, true))) return rc;
         if ((rc = mark_search_start(p))) return rc;
         k.init = captured ? 0 : p->needs_init ? 2 : 1;
         k.barrier_sel = p->barrier_sel;
