@@ -939,13 +939,7 @@ int b40c_bfs_set_stream(b40c_bfs_problem *p, void *stream)
 {
     b40c::clear_error();
     if (!p) return b40c::fail(B40C_ERROR_INVALID_VALUE, "null problem");
-    const cudaStream_t next = stream ? (cudaStream_t)stream : p->own_stream;
-    if (next != p->stream && p->reset_pending) {
-        DeviceGuard guard(p->device);
-        CUDA_TRY(cudaStreamSynchronize(p->stream), "reset synchronize");
-        p->reset_pending = false;
-    }
-    p->stream = next;
+    p->stream = stream ? (cudaStream_t)stream : p->own_stream;
     return B40C_SUCCESS;
 }
 
@@ -981,9 +975,10 @@ int b40c_bfs_problem_reset(b40c_bfs_problem *p, int frontier_type, double queue_
     CUDA_TRY(cudaMemcpyAsync(p->d_mask, p->d_iso, sizeof(uint32_t) * p->mask_words, cudaMemcpyDeviceToDevice,
                              p->stream),
              "mask reset");
-    // the search that follows is ordered after the fills on the handle's stream
-    // (a wait here cost the smallest search call 9 of its 98 us)
-    p->reset_pending = true;
+    // the caller may go on anywhere: on another stream (b40c_bfs_set_stream, the
+    // device view) or with a replay of a captured search (the wait costs the
+    // smallest search call 9 us; the order of one stream cannot stand in for it)
+    CUDA_TRY(cudaStreamSynchronize(p->stream), "reset synchronize");
     p->needs_init = false;
     return B40C_SUCCESS;
 }

@@ -106,7 +106,6 @@ struct b40c_bfs_problem {
     bool timed = false;
     bool needs_init = true;  // labels/mask dirty since the last reset
     int barrier_sel = 0;     // launch barrier of the next persistent search
-    bool reset_pending = false;  // a reset's fills may still run on `stream` (b40c_bfs_set_stream waits for them)
     bool queues_edges = false;  // the last search's queue total is its levels' edges (fused edge strategies)
     // CUDA graphs of whole searches (ENACT_GRAPH), one per strategy, rebuilt
     // when the kernel parameters (buffers, policy) or the grid change

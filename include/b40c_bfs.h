@@ -205,7 +205,7 @@ int b40c_bfs_problem_create(const int32_t *h_row_offsets, const int32_t *h_colum
 int b40c_bfs_problem_destroy(b40c_bfs_problem *problem);
 
 /* Orders the handle's work on a caller stream (a cudaStream_t); NULL restores
- * the handle's own stream.  Waits for a reset still running on the old one. */
+ * the handle's own stream.  Work queued before stays on the old one. */
 int b40c_bfs_set_stream(b40c_bfs_problem *problem, void *cuda_stream);
 
 /* Device bytes the handle holds now (CSR copy, labels, masks, queues, batch
@@ -215,8 +215,8 @@ int b40c_bfs_problem_device_bytes(b40c_bfs_problem *problem, int64_t *bytes);
 
 /* CsrProblem::Reset (csr_problem.cuh:547-750): (re)allocates the frontier
  * queues for frontier_type at queue_sizing x n (vertex) or x m (edge)
- * elements, and initialises labels to -1 and the visited mask to 0, in order on
- * the handle's stream (it does not wait for the fills). */
+ * elements, and initialises labels to -1 and the visited mask to 0; the fills
+ * are done when it returns. */
 int b40c_bfs_problem_reset(b40c_bfs_problem *problem, int frontier_type, double queue_sizing);
 
 /* Enact{Fused,Iterative}Search / EnactSearch (enactor_contract_expand.cuh:262,419;
