@@ -352,8 +352,10 @@ int sort_passes(const int32_t *d_rows, const int32_t *d_cols, int64_t nodes, int
     const int64_t per_cta = (tiles + ctas - 1) / ctas * tile;
     const int grid = (int)((edges + per_cta - 1) / per_cta);
     const size_t smem = scatter_smem<THREADS, PER>(bins);
+    // (the limit belongs to the kernel: every conversion sets the same one, for the
+    // widest digit, so none running beside it finds its own launch above the limit)
     CUDA_TRY(cudaFuncSetAttribute(scatter_kernel<THREADS, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem),
+                                  (int)scatter_smem<THREADS, PER>(kMaxBins)),
              "smem attribute");
     const int32_t *kin = d_rows, *vin = d_cols;
     for (int pass = 0; pass < passes; pass++) {

@@ -81,6 +81,34 @@ def test_columns_converted_in_place(n):
     assert np.array_equal(d_c.cpu().numpy(), want_ci)
 
 
+def test_conversions_from_several_threads():
+    """Digits of different widths at the same time, in short and in long tiles: the
+    kernels' shared memory differs with the width."""
+    import threading
+    import torch
+    cases = []
+    for n, m in ((2048, 100_000), (40, 100_000), (1 << 22, 70_000), (2048, 148 * 16384), (40, 148 * 16384)):
+        rng = np.random.default_rng(n + m)
+        rows, cols = rng.integers(0, n, m), rng.integers(0, n, m)
+        cases.append((n, rows, cols, _host_csr(n, rows, cols)))
+    wrong = []
+
+    def work(n, rows, cols, want):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(60):
+                rc, ro, ci = _device(n, rows, cols)
+                if rc != 0 or not np.array_equal(ro, want[0]) or not np.array_equal(ci, want[1]):
+                    wrong.append((n, rows.size, rc))
+                    return
+
+    threads = [threading.Thread(target=work, args=c) for c in cases]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 def test_rejects_ids_out_of_range():
     rows = np.array([0, 1, 5], np.int32)
     cols = np.array([1, 2, 0], np.int32)
