@@ -292,11 +292,14 @@ __global__ void row_offsets_kernel(const int32_t *keys, int64_t m, int64_t n, in
     }
 }
 
-// Temporary memory of a conversion, stream-ordered, from one pool per device.
-// A conversion of 16 M edges needs 200 MB, and mapping that anew costs more
-// than the sort; the pool keeps up to kPoolKeep bytes between calls (more is
-// given back at the next synchronize) and is safe with any thread and stream.
-constexpr uint64_t kPoolKeep = 256ull << 20;
+// Temporary memory of a conversion, stream-ordered, from one pool per device that
+// is safe with any thread and stream.  A conversion of 16 M edges needs 200 MB, and
+// mapping that anew costs more than the sort; the pool keeps up to kPoolKeep bytes
+// between calls.  A conversion frees its workspace ahead of its last wait, so what is
+// kept is settled when it returns: more than kPoolKeep goes back to the device
+// there, the rest with b40c_coo_release_memory, after a problem_create_coo and when an
+// allocation of this library runs short.
+constexpr uint64_t kPoolKeep = 512ull << 20;
 constexpr int kMaxDevices = 64;
 static cudaMemPool_t g_pool[kMaxDevices];
 static std::mutex g_pool_mutex;
@@ -336,9 +339,20 @@ struct Workspace {
     unsigned char *p = nullptr;
     cudaStream_t s;
     explicit Workspace(cudaStream_t stream) : s(stream) {}
+    // Before the caller's last wait: the pool counts freed memory as its own only
+    // once the host has seen the free done.
+    cudaError_t release()
+    {
+        void *q = p;
+        p = nullptr;
+        return q ? cudaFreeAsync(q, s) : cudaSuccess;
+    }
     ~Workspace()
     {
-        if (p) cudaFreeAsync(p, s);
+        if (!p) return;
+        release();  // a failed conversion
+        cudaStreamSynchronize(s);
+        cudaGetLastError();
     }
 };
 
@@ -457,6 +471,7 @@ int coo_to_csr_device(const int32_t *d_rows, const int32_t *d_cols, int64_t node
     CUDA_TRY(cudaGetLastError(), "row offsets launch");
     int32_t h_bad = 0;
     CUDA_TRY(cudaMemcpyAsync(&h_bad, flag, sizeof(int32_t), cudaMemcpyDeviceToHost, s), "flag read");
+    CUDA_TRY(ws.release(), "conversion workspace release");
     CUDA_TRY(cudaStreamSynchronize(s), "conversion");
     if (h_bad) return b40c::fail(B40C_ERROR_INVALID_VALUE, "COO vertex id out of [0, %lld)", (long long)nodes);
     return B40C_SUCCESS;
@@ -485,6 +500,19 @@ int b40c_coo_to_csr_device(const int32_t *d_rows, const int32_t *d_cols, int64_t
     }
     return coo_to_csr_device(d_rows, d_cols, nodes, edges, d_row_offsets, d_column_indices,
                              (cudaStream_t)cuda_stream, device, sms);
+}
+
+int b40c_coo_release_memory(int device)
+{
+    b40c::clear_error();
+    int count = 0;
+    if (cudaGetDeviceCount(&count) != cudaSuccess || count < 1) {
+        cudaGetLastError();
+        return b40c::fail(B40C_ERROR_NO_DEVICE, "no CUDA device");
+    }
+    if (device < 0 || device >= count) return b40c::fail(B40C_ERROR_INVALID_VALUE, "device %d", device);
+    release_conversion_memory(device);
+    return B40C_SUCCESS;
 }
 
 int b40c_bfs_problem_create_coo(const int32_t *h_rows, const int32_t *h_cols, int64_t nodes, int64_t edges,

@@ -406,9 +406,14 @@ int b40c_build_grid3d(int32_t width, int pinned, b40c_csr *out);
  * into d_row_offsets[nodes + 1] and d_column_indices[edges] with rows in
  * input order (a stable radix sort by row).  Ids outside [0, nodes) return
  * B40C_ERROR_INVALID_VALUE.  Synchronous on cuda_stream; temporary device
- * memory of about 16 bytes per edge is allocated and freed inside. */
+ * memory of up to 16 bytes per edge comes from a pool of the library's own, which
+ * keeps at most 512 MB per device between calls. */
 int b40c_coo_to_csr_device(const int32_t *d_rows, const int32_t *d_cols, int64_t nodes, int64_t edges,
                            int32_t *d_row_offsets, int32_t *d_column_indices, void *cuda_stream);
+
+/* Gives back to the device what the conversions' pool keeps between calls (the
+ * next conversion maps its memory anew); conversions in progress are unaffected. */
+int b40c_coo_release_memory(int device);
 
 /* A problem handle built from a host COO edge list (FromCoo + FromHostProblem
  * in one step): the list is uploaded and converted on the GPU. */

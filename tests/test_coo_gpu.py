@@ -109,6 +109,48 @@ def test_conversions_from_several_threads():
     assert not wrong
 
 
+def _in_use():
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def test_conversion_memory_is_bounded_and_given_back():
+    """60 M edges need 720 MB of workspace: at most 512 MB stay when the call returns
+    (mapped in steps of 32 MB), nothing after the release."""
+    import torch
+    n, m = 1 << 20, 60_000_000
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    _device(n, np.arange(1000), np.arange(1000))
+    assert N.lib().b40c_coo_release_memory(0) == 0
+    base = _in_use()
+    r = torch.randint(0, n, (m,), generator=gen, device="cuda", dtype=torch.int32)
+    ro = torch.empty(n + 1, dtype=torch.int32, device="cuda")
+    ci = torch.empty(m, dtype=torch.int32, device="cuda")
+    assert N.lib().b40c_coo_to_csr_device(r.data_ptr(), r.data_ptr(), n, m, ro.data_ptr(), ci.data_ptr(),
+                                          torch.cuda.current_stream().cuda_stream) == 0
+    del r, ro, ci
+    assert _in_use() - base <= (512 + 32) << 20
+    assert N.lib().b40c_coo_release_memory(0) == 0
+    assert _in_use() - base <= 8 << 20
+    assert N.lib().b40c_coo_release_memory(99) == N.ERROR_INVALID_VALUE
+
+
+def test_problem_from_coo_keeps_no_conversion_memory():
+    rng = np.random.default_rng(4)
+    n, m = 100_000, 16_000_000
+    rows, cols = rng.integers(0, n, m), rng.integers(0, n, m)
+    CsrProblem.from_coo(rows[:1000], cols[:1000], n).Destroy()
+    base = _in_use()
+    p = CsrProblem.from_coo(rows, cols, n)
+    held = C.c_int64()
+    N.check(N.lib().b40c_bfs_problem_device_bytes(p.handle, C.byref(held)))
+    assert _in_use() - base <= held.value + (32 << 20)  # (192 MB of workspace)
+    p.Destroy()
+
+
 def test_rejects_ids_out_of_range():
     rows = np.array([0, 1, 5], np.int32)
     cols = np.array([1, 2, 0], np.int32)
