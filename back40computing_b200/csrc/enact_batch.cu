@@ -149,7 +149,7 @@ int enact_batch(b40c_bfs_problem *p, const int32_t *sources, const int32_t *limi
                         : block == 512 ? sizeof(dev::MsSmem<512>)
                                        : sizeof(dev::MsSmem<256>);
     int grid = 0;
-    if ((rc = persistent_grid(p, kern, pol, max_grid, smem, &grid))) return rc;
+    if ((rc = persistent_grid(p, kern, pol, max_grid, smem, smem, &grid))) return rc;
     p->enact_events[0] = p->ev0;
     p->enact_events[1] = p->ev1;
     CUDA_TRY(cudaEventRecord(p->ev0, p->stream), "event record");

@@ -38,7 +38,7 @@ int enact_phases_t(b40c_bfs_problem *p, int strategy, int mode, int32_t src, int
     const void *kern = (const void *)dev::edge_kernel<B, PRED>;
     const size_t smem = kernel_smem<dev::ExpandSmem<B, PRED>>(pol);
     int grid = 0;
-    if ((rc = persistent_grid(p, kern, pol, max_grid, smem, &grid))) return rc;
+    if ((rc = persistent_grid(p, kern, pol, max_grid, smem, kernel_smem_limit<B, PRED>(), &grid))) return rc;
     if ((rc = begin_enact(p, src, depth_limit))) return rc;
     if ((rc = begin_instrumented(p))) return rc;
 

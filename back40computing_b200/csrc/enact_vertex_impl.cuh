@@ -56,7 +56,7 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
         if (lists_kernel) kern = (const void *)dev::ec_kernel<256, false, true>;
     const size_t smem = kernel_smem<dev::ExpandSmem<B, PRED>>(pol);
     int grid = 0;
-    if ((rc = persistent_grid(p, kern, pol, max_grid, smem, &grid))) return rc;
+    if ((rc = persistent_grid(p, kern, pol, max_grid, smem, kernel_smem_limit<B, PRED>(), &grid))) return rc;
     if ((rc = begin_enact(p, src, depth_limit, mode == B40C_ENACT_FUSED))) return rc;
     if ((rc = begin_instrumented(p))) return rc;
     if (mode == B40C_ENACT_GRAPH) {

@@ -19,6 +19,16 @@ inline size_t kernel_smem(const b40c_bfs_policy &pol)
            (pol.warp_contract > 0 && pol.threads > 256 ? (size_t)(pol.threads / 32) * dev::kWarpTableBytes : 0);
 }
 
+// The most any policy makes of it.  A kernel's limit on dynamic shared memory is
+// shared by all handles and threads, so it is this for every launch: one set for
+// a launch's own policy could be lowered by another thread's before the launch.
+template <int B, bool PRED>
+constexpr size_t kernel_smem_limit()
+{
+    return ((sizeof(dev::ExpandSmem<B, PRED>) + 15) & ~size_t(15)) + (sizeof(uint32_t) << kHistLog) +
+           dev::kBuPrefetchBytes + (B > 256 ? (size_t)(B / 32) * dev::kWarpTableBytes : 0);
+}
+
 // Grid of the set-up kernel: the full label/mask initialisation is a
 // grid-stride fill, the source-only set-up a single CTA.
 inline int init_grid(b40c_bfs_problem *p, bool full)

@@ -13,8 +13,7 @@
 // run as one persistent cooperative grid; only the storage differs.
 #include <mutex>
 
-#include "bfs_kernels.cuh"
-#include "problem.h"
+#include "launch_common.cuh"
 
 namespace b40c {
 namespace noalloc {
@@ -24,9 +23,7 @@ constexpr int64_t kMaxEdges = 1 << 22;  // 4,194,304 directed edges
 constexpr int kThreads = 256;
 // Graphs of up to this many edges run one 512-thread CTA per SM (default_launch's
 // rule; us per call against four of 256: random 20,000 x 8 126 / 94, 80,707 x 2
-// 134 / 119), larger ones four of 256, their large levels warp by warp.  Neither
-// asks for shared memory past the kernel's own arrays, so no other search of the
-// same kernel can leave its limit too low for these launches.
+// 134 / 119), larger ones four of 256, their large levels warp by warp.
 constexpr int64_t kSmallEdges = 1 << 21;
 constexpr int kSmallThreads = 512;
 
@@ -81,9 +78,12 @@ static int set_up(int device, DeviceSetup **out)
         const void *small = (const void *)dev::ec_kernel<kSmallThreads, false, false, false>;
         const size_t smem = sizeof(dev::ExpandSmem<kThreads, false>);
         const size_t small_smem = sizeof(dev::ExpandSmem<kSmallThreads, false>);
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // (the limits that the other searches of these kernels set)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)rt::kernel_smem_limit<kThreads, false>());
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem);
+            e = cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)rt::kernel_smem_limit<kSmallThreads, false>());
         int per_sm = 0, small_per_sm = 0, sms = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem);
         if (e == cudaSuccess)

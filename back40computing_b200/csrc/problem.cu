@@ -397,11 +397,12 @@ __global__ void stage_results_kernel(const int32_t *labels, int32_t *stage, int6
 
 
 int persistent_grid(b40c_bfs_problem *p, const void *kernel, const b40c_bfs_policy &pol, int max_grid,
-                            size_t smem, int *grid)
+                            size_t smem, size_t smem_limit, int *grid)
 {
     int per_sm = 0;
-    // (the attribute belongs to the kernel, not to this handle: set for every launch)
-    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
+    // (the attribute belongs to the kernel in this context, not to this handle)
+    CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit),
+             "smem attribute");
     for (const auto &o : p->occupancy)
         if (o.kernel == kernel && o.threads == pol.threads && o.smem == smem) per_sm = o.per_sm;
     if (per_sm == 0) {

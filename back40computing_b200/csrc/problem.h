@@ -173,8 +173,9 @@ b40c_bfs_policy default_policy(int strategy);
 int resolve_policy(int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *out);
 int read_state(b40c_bfs_problem *p);
 int check_state_errors(b40c_bfs_problem *p);
+// `smem` of this launch, `smem_limit` the same for every launch of the kernel.
 int persistent_grid(b40c_bfs_problem *p, const void *kernel, const b40c_bfs_policy &pol, int max_grid, size_t smem,
-                    int *grid);
+                    size_t smem_limit, int *grid);
 int finish_timing(b40c_bfs_problem *p);
 int begin_instrumented(b40c_bfs_problem *p);
 void free_graphs(b40c_bfs_problem *p);
