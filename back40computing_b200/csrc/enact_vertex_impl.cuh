@@ -45,8 +45,10 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
     const bool lists_kernel = direction_opt && !PRED && pol.bottom_up_list > 0;
     // plain expand-contract searches (and directed graphs) never go bottom-up:
     // they run the top-down-only variants; list mode is built for 256-thread CTAs
-    // only, and a sub-grid threshold asks for them too
-    const bool subgrid = mode == B40C_ENACT_FUSED && pol.subgrid_frontier_edges > 0;
+    // only, and a sub-grid threshold asks for them too (not of the edge-frontier
+    // strategies, whose policies may carry one with any CTA size)
+    const bool subgrid =
+        mode == B40C_ENACT_FUSED && pol.subgrid_frontier_edges > 0 && edge_limit == INT32_MAX;
     if (B != 256 && (lists_kernel || subgrid))
         return b40c::fail(B40C_ERROR_INVALID_VALUE,
                           "policy.threads %d: bottom-up list mode and the sub-grid phase need 256", B);

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 import oracle
-from back40computing_b200 import CsrGraph, CsrProblem, BuildGrid3dGraph, search, EXPAND_CONTRACT, DIRECTION_OPTIMIZING
+from back40computing_b200 import (CsrGraph, CsrProblem, BuildGrid3dGraph, search, EXPAND_CONTRACT, CONTRACT_EXPAND,
+                                  TWO_PHASE, HYBRID, DIRECTION_OPTIMIZING)
 from back40computing_b200 import _native as N
 from back40computing_b200.bfs import ENACTORS
 
@@ -114,3 +115,19 @@ def test_levels_of_more_edges_than_vertices(n, degree, threads, precheck):
                 assert np.array_equal(want[got[reached]] + 1, want[reached])
             else:
                 assert oracle.compare_labels(got, want) == -1
+
+
+@pytest.mark.parametrize("strategy", [CONTRACT_EXPAND, TWO_PHASE, HYBRID])
+@pytest.mark.parametrize("threads", [128, 256, 512])
+def test_edge_strategies_take_a_subgrid_threshold(strategy, threads):
+    """With any CTA size, where the vertex-frontier strategies ask for 256 threads."""
+    g = _graph("lattice")
+    p = CsrProblem.from_graph(g)
+    pol = N.Policy()
+    pol.threads, pol.subgrid_frontier_edges = threads, 3000
+    want = oracle.bfs(g.row_offsets, g.column_indices, 0)[0]
+    assert oracle.compare_labels(search(p, 0, strategy=strategy, policy=pol), want) == -1
+    if threads != 256:
+        with pytest.raises(N.B40cError):
+            search(p, 0, strategy=EXPAND_CONTRACT, policy=pol)
+    p.Destroy()
