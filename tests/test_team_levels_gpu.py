@@ -131,3 +131,16 @@ def test_edge_strategies_take_a_subgrid_threshold(strategy, threads):
         with pytest.raises(N.B40cError):
             search(p, 0, strategy=EXPAND_CONTRACT, policy=pol)
     p.Destroy()
+
+
+@pytest.mark.parametrize("kind", ["lattice", "hub"])
+@pytest.mark.parametrize("strategy", [EXPAND_CONTRACT, DIRECTION_OPTIMIZING])
+@pytest.mark.parametrize("mode", [N.ENACT_FUSED, N.ENACT_GRAPH])
+def test_host_mapped_graph(kind, strategy, mode):
+    """Levels of a CSR read from host memory take their winners' rows only."""
+    g = _graph(kind)
+    want = oracle.bfs(g.row_offsets, g.column_indices, 0)[0]
+    p = CsrProblem.from_graph(g, stream_from_host=True)
+    for _ in range(2):
+        assert oracle.compare_labels(search(p, 0, strategy=strategy, mode=mode), want) == -1
+    p.Destroy()
