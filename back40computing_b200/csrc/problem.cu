@@ -286,8 +286,10 @@ int resolve_policy(int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *out
 //  * one CTA per SM while the graph is small, where a level's cost is its barriers:
 //    direction-optimizing searches up to 2^19 vertices (R-MAT 16 63 / 55, R-MAT
 //    19 69 / 64, but random 10^6 112 / 130), top-down ones up to 2^21 edges
-//    (R-MAT 13 and random 20,000 107 / 67 and 100 / 62, R-MAT 17 88 / 92).
-void default_launch(const b40c_bfs_problem *p, int strategy, const b40c_bfs_policy *in, b40c_bfs_policy *pol)
+//    (R-MAT 13 and random 20,000 107 / 67 and 100 / 62, R-MAT 17 88 / 92).  Per-level
+//    expand-contract launches are sized level by level (enact_ec_t).
+void default_launch(const b40c_bfs_problem *p, int strategy, int mode, const b40c_bfs_policy *in,
+                    b40c_bfs_policy *pol)
 {
     if ((!in || in->threads == 0) && pol->bottom_up_list <= 0 && pol->subgrid_frontier_edges <= 0 &&
         pol->warp_contract > 0) {
@@ -297,8 +299,9 @@ void default_launch(const b40c_bfs_problem *p, int strategy, const b40c_bfs_poli
     }
     if (!in || in->ctas_per_sm == 0) {
         const bool small = strategy == B40C_DIRECTION_OPTIMIZING ? p->nodes <= (int64_t)1 << 19
-                                                                 : p->edges <= (int64_t)1 << 21;
-        if (small && pol->threads == 512) pol->ctas_per_sm = 1;
+                                                                 : p->edges <= kSmallGraphEdges;
+        const bool level_by_level = strategy == B40C_EXPAND_CONTRACT && mode == B40C_ENACT_ITERATIVE;
+        if (small && pol->threads == 512 && !level_by_level) pol->ctas_per_sm = 1;
     }
 }
 
@@ -994,7 +997,7 @@ int b40c_bfs_enact_limited(b40c_bfs_problem *p, int strategy, int mode, int32_t 
     b40c_bfs_policy pol;
     int rc = resolve_policy(strategy, policy, &pol);
     if (rc) return rc;
-    default_launch(p, strategy, policy, &pol);
+    default_launch(p, strategy, mode, policy, &pol);
     DeviceGuard guard(p->device);
     p->timed = false;
     p->queues_edges = false;

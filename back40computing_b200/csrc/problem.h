@@ -194,6 +194,9 @@ int run_graph(b40c_bfs_problem *p, int slot, const KernelNode &init, KernelNode 
 
 // enactors
 // `edge_limit`: the largest level accepted, in edges (fused edge-frontier strategies)
+// Top-down searches of graphs of up to this many edges run one CTA per SM unless the
+// caller says otherwise (default_launch).
+constexpr int64_t kSmallGraphEdges = (int64_t)1 << 21;
 int enact_vertex(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b40c_bfs_policy &pol,
                  int32_t depth_limit, bool direction_optimizing, int32_t edge_limit = INT32_MAX);
 int check_symmetric(b40c_bfs_problem *p);
