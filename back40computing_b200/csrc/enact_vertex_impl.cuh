@@ -98,9 +98,9 @@ int enact_ec_t(b40c_bfs_problem *p, int mode, int32_t src, int max_grid, const b
         if ((rc = mark_search_start(p))) return rc;
         // one launch per level; the host reads the next frontier's size.  On a small
         // graph one CTA per SM, but a level nearly all of whose edges meet visited
-        // vertices is bound by its tests and takes what fits (R-MAT 16 x 5, 299 thousand
-        // edges with 8 thousand left: 30.4 us a level with one, 28.2 with two; the level
-        // before it, with as many left as it has, 30.8 and 36.3)
+        // vertices is bound by its tests and takes what fits (us per level with one and
+        // with two: R-MAT 16 x 8, 741 thousand edges with 24 thousand left, 37 and 26;
+        // R-MAT 16 x 5, 344 thousand with 307 thousand left, 31 and 36)
         const bool small = B == 512 && pol.ctas_per_sm == 0 && p->edges <= kSmallGraphEdges;
         for (int level = 0;; level++) {
             if ((rc = read_state(p))) return rc;
