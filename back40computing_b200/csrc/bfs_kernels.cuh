@@ -263,9 +263,9 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
     unsigned word[U];
     // more items than vertices: most lose, and all meet on few mask and row lines, so
     // only winners read their rows (random 2154 x 16, a level of 43 thousand edges
-    // launched by itself: 15.1 -> 5.5 us)
-    const bool busy = items > p.nodes;
-    const bool late_rows = busy || !p.bulk_ok;
+    // launched by itself: 15.1 -> 5.5 us); a host-mapped CSR's rows come over the host
+    // link, in every level for winners only (grid3d-60 as a graph 3.27 -> 2.64 ms)
+    const bool busy = items > p.busy_items;
     const bool precheck = p.precheck && (items >= kPrecheckItems || busy) && !(LISTS && s.ul_in >= 0);
     uint32_t *hist = s.hist;
 #pragma unroll
@@ -299,9 +299,7 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
         }
     } else {
         // the rows are loaded beside the test-and-set, for losers too: a level
-        // of this size waits for round trips, not for their bandwidth (but a host-mapped
-        // CSR's rows come over the host link, and for winners only: grid3d-60 as a graph
-        // 3.27 -> 2.64 ms, fused 1.80 -> 1.49)
+        // of this size waits for round trips, not for their bandwidth
         unsigned old[U];
 #pragma unroll
         for (int t = 0; t < U; t++) {
@@ -313,7 +311,7 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
 #pragma unroll
         for (int t = 0; t < U; t++) {
             r0[t] = r1[t] = 0;
-            if (go[t] && !late_rows) {
+            if (go[t] && !busy) {
                 r0[t] = ld_ro(p.row_offsets + v[t]);
                 r1[t] = ld_ro(p.row_offsets + v[t] + 1);
             }
@@ -321,7 +319,7 @@ __device__ __forceinline__ void discover_batch(const BfsParams &p, ExpandSmem<B,
 #pragma unroll
         for (int t = 0; t < U; t++) {
             found[t] = !((old[t] >> (v[t] & 31)) & 1u);
-            if (found[t] && late_rows) {
+            if (found[t] && busy) {
                 r0[t] = ld_ro(p.row_offsets + v[t]);
                 r1[t] = ld_ro(p.row_offsets + v[t] + 1);
             }
@@ -2264,9 +2262,8 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
     // pre-check (through L1), and only winners read their rows (random 20,000 x 8,
     // 237 thousand edges, 256-thread CTAs: 24.4 -> 11.8 us)
     // (as do all levels of a host-mapped CSR, whose rows come over the host link)
-    bool busy = s.E > p.nodes;
+    bool busy = s.E > p.busy_items;
     for (int run = 0;; run++) {
-        const bool late_rows = busy || !p.bulk_ok;
         if (E > 0) stamp(p, level, 0);
         fill_owners<B>(s, n);
         __syncthreads();
@@ -2313,7 +2310,7 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
 #pragma unroll
             for (int t = 0; t < PER; t++) {
                 r0[t] = deg[t] = 0;
-                if (v[t] >= 0 && !late_rows) {
+                if (v[t] >= 0 && !busy) {
                     r0[t] = ld_ro(p.row_offsets + v[t]);
                     deg[t] = ld_ro(p.row_offsets + v[t] + 1);
                 }
@@ -2322,7 +2319,7 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
             for (int t = 0; t < PER; t++)
                 if (!((old[t] >> (v[t] & 31)) & 1u)) {
                     found |= 1u << t;
-                    if (late_rows) {
+                    if (busy) {
                         r0[t] = ld_ro(p.row_offsets + v[t]);
                         deg[t] = ld_ro(p.row_offsets + v[t] + 1);
                     }
@@ -2380,7 +2377,7 @@ __device__ __forceinline__ void team_phase(const BfsParams &p, ExpandSmem<B, PRE
             (BU && team > 1 &&
              choose_bottom_up(p, false, n_all, E_all, visited + (unsigned long long)(unsigned)E_all)))
             break;
-        busy = E_all > p.nodes;
+        busy = E_all > p.busy_items;
         visited += (unsigned long long)(unsigned)E_all;
         queued += (unsigned long long)(unsigned)n_all;
         if (run == 0 && blockIdx.x == 0) {

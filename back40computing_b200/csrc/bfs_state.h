@@ -146,6 +146,8 @@ struct BfsParams {
     int32_t cta_thresh;
     int32_t warp_cull;
     int32_t precheck;
+    int32_t busy_items;       // passes of more items than this pre-check, and only winners read their rows:
+                              // the vertices, or -1 for a host-mapped CSR
     int32_t persistent;       // 1: loop over levels with the grid barrier
     int32_t skip_arrival_cta; // test-only fault injection: this CTA never arrives (-1 = off)
     uint32_t late_start_ns;   // test-only: CTAs other than 0 of a persistent launch start this late (0 = off)

@@ -168,6 +168,7 @@ extern "C" int b40c_bfs_search_noalloc(const int32_t *d_row_offsets, const int32
     k.cta_thresh = 512;
     k.warp_cull = 0;
     k.precheck = 1;
+    k.busy_items = (int32_t)nodes;
     k.edge_limit = INT32_MAX;
     k.persistent = 1;
     k.skip_arrival_cta = -1;

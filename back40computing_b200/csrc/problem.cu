@@ -158,6 +158,7 @@ BfsParams make_params(b40c_bfs_problem *p, const b40c_bfs_policy &pol)
     k.cta_thresh = pol.cta_gather_threshold;
     k.warp_cull = pol.warp_cull;
     k.precheck = pol.bitmask_precheck > 0 ? pol.bitmask_precheck : 0;  // -1 (off) must not read as true
+    k.busy_items = p->stream_from_host ? -1 : (int32_t)p->nodes;
     k.edge_limit = INT32_MAX;
     k.persistent = 0;
     k.skip_arrival_cta = -1;
