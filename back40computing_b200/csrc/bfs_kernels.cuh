@@ -494,6 +494,12 @@ __device__ __forceinline__ void cta_range(int n, int part, int parts, int &rs, i
     re = (b == G - 1) ? n : (int)((long long)n * (b + 1) / G / kChunkGrain * kChunkGrain);
 }
 
+// Warp-autonomous passes are taken by levels with at least a full sub-round
+// of work per CTA: in smaller ones (the first levels from a hub, which
+// discover most of what they touch) a warp would flush its output after
+// nearly every slice, and the CTA-wide sub-rounds measured 3x faster there.
+__device__ __forceinline__ bool warp_sized(int items) { return items >= (int)gridDim.x * kChunkMax; }
+
 // The run tables' position -> entry map (s.own) from the entries' first
 // positions s.rel[0..n], s.rel[n] the end: short lists by their lane, long ones
 // by the whole warp (against a binary search per thread: 0.7 -> 0.3 us of a
@@ -515,6 +521,35 @@ __device__ __forceinline__ void fill_owners(Smem &s, int n)
             todo &= todo - 1;
             const int a = __shfl_sync(0xffffffffu, lo, L), b = __shfl_sync(0xffffffffu, hi, L);
             for (int x = a + lane; x < b; x += 32) s.own[x] = (uint16_t)(jb + L);
+        }
+    }
+}
+
+// The same with a binary search per thread: thread t resolves positions
+// [t * PER, t * PER + PER) of len.  A call of its own: inlined, it cost the resident
+// levels of the same kernel 9 % (grid2d-1000 4.65 -> 5.2 ms).
+template <int B, typename Smem>
+__device__ __noinline__ void search_owners(Smem &s, int n, int len)
+{
+    constexpr int PER = kChunkMax / B;
+    const int x0 = threadIdx.x * PER;
+    if (x0 >= len) return;
+    int lo = 0, hi = n - 1;  // last j with rel[j] <= x0
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (s.rel[mid] <= x0) lo = mid; else hi = mid - 1;
+    }
+    int j = lo;
+    int next = s.rel[j + 1];
+#pragma unroll
+    for (int t = 0; t < PER; t++) {
+        const int x = x0 + t;
+        if (x < len) {
+            while (x >= next) {
+                j++;
+                next = s.rel[j + 1];
+            }
+            s.own[x] = (uint16_t)j;
         }
     }
 }
@@ -633,7 +668,14 @@ __device__ __forceinline__ void expand_range(const BfsParams &p, const VertexFro
             }
         } else {
             __syncthreads();  // rel[k] is written
-            fill_owners<B>(s, k);
+            // levels of several sub-rounds per CTA are bound by instructions, not by
+            // their round trips: the searches cost fewer (R-MAT 22 expand-contract without
+            // warp-by-warp levels, us: 256 threads 1850 / 1790, 512 threads 2555 / 2316, but
+            // 128 threads 2870 / 2944)
+            if (B >= 256 && warp_sized(E))
+                search_owners<B>(s, k, len);
+            else
+                fill_owners<B>(s, k);
         }
         if (!__syncthreads_and(staged)) {
             // the copy did not land in time: report it, give the copy still in
@@ -812,12 +854,6 @@ __device__ __forceinline__ void warp_emit(const BfsParams &p, const int32_t *bv,
         }
     }
 }
-
-// Warp-autonomous passes are taken by levels with at least a full sub-round
-// of work per CTA: in smaller ones (the first levels from a hub, which
-// discover most of what they touch) a warp would flush its output after
-// nearly every slice, and the CTA-wide sub-rounds measured 3x faster there.
-__device__ __forceinline__ bool warp_sized(int items) { return items >= (int)gridDim.x * kChunkMax; }
 
 // Warp-autonomous passes deal their slices over every warp of the grid,
 // warp-major (slice k goes to warp k / gridDim of CTA k % gridDim, then
