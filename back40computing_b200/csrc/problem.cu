@@ -998,6 +998,9 @@ int b40c_bfs_enact_limited(b40c_bfs_problem *p, int strategy, int mode, int32_t 
     b40c_bfs_policy pol;
     int rc = resolve_policy(strategy, policy, &pol);
     if (rc) return rc;
+    // (a fused edge-frontier search has no contract and expand passes for this to
+    // choose between, and would lose by CTA-wide levels: R-MAT 22 1790 / 813 us)
+    if (mode == B40C_ENACT_FUSED && strategy >= B40C_CONTRACT_EXPAND && strategy <= B40C_HYBRID) pol.warp_contract = 1;
     default_launch(p, strategy, mode, policy, &pol);
     DeviceGuard guard(p->device);
     p->timed = false;

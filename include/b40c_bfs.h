@@ -149,7 +149,8 @@ typedef struct b40c_bfs_policy {
                                       the level, dealt over every warp of the grid, with no CTA barriers,
                                       and sends its winners to the vertex frontier in flushes of its own
                                       (one packed atomic each; default), -1 = CTA-wide sub-rounds
-                                      (queue_allocation applies) */
+                                      (queue_allocation applies); fused searches of the edge-frontier
+                                      strategies, which have no such passes, always go warp by warp */
     int32_t warp_bottom_up;        /* direction-optimizing fused searches, the first bottom-up level of a
                                       run when it only counts its discoveries: 1 = each warp takes blocks
                                       of vertex ids dealt over every warp of the grid, with no CTA
