@@ -215,11 +215,11 @@ def main(argv=None):
     out = load_cache(args.out) if os.path.exists(args.out) else {}
     out.setdefault("classes", {})
     out["device"] = torch.cuda.get_device_name(0)
-    out["generated"] = time.strftime("%Y-%m-%dT%H:%M:%SZ", time.gmtime())
-    out["how"] = ("coordinate search over SEARCH_SPACE "
-                  + (f"of the knobs {args.knobs} from the cached policy" if args.knobs else "from the library defaults")
-                  + "; cost = mean device time per search (per batch for 'batched') summed over the class's "
-                  f"representatives; quick={args.quick}")
+    # a run may tune some rows only: each row says when and how it was measured
+    how = ("coordinate search over SEARCH_SPACE "
+           + (f"of the knobs {args.knobs} from the cached policy" if args.knobs else "from the library defaults")
+           + "; cost = mean device time per search (per batch for 'batched') summed over the class's "
+           f"representatives; quick={args.quick}")
     for cls in args.classes.split(","):
         for kind in args.kinds.split(","):
             print(f"[{cls} / {kind}]", flush=True)
@@ -228,6 +228,7 @@ def main(argv=None):
             best, base, t = tune_class(reps[cls], kind, start=start, knobs=knobs)
             out["classes"].setdefault(cls, {})[kind] = {
                 "policy": best, "default_ms": base, "tuned_ms": t,
+                "generated": time.strftime("%Y-%m-%dT%H:%M:%SZ", time.gmtime()), "how": how,
                 "graphs": [name for name, _ in reps[cls]]}
             print(f"  default {base:.3f} ms -> tuned {t:.3f} ms  {best}", flush=True)
             with open(args.out, "w") as f:

@@ -53,3 +53,12 @@ def test_committed_cache_is_well_formed():
             for knob, v in entry["policy"].items():
                 assert knob in autotune.SEARCH_SPACE and v in autotune.SEARCH_SPACE[knob]
             assert entry["tuned_ms"] <= entry["default_ms"]
+
+
+def test_every_committed_row_says_when_and_how():
+    """Rows are tuned in different runs: no date or method above them speaks for all."""
+    cache = autotune.load_cache()
+    assert not {"generated", "how"} & set(cache)
+    for kinds in cache["classes"].values():
+        for entry in kinds.values():
+            assert entry["generated"].startswith("20") and "SEARCH_SPACE" in entry["how"]
