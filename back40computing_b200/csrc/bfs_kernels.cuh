@@ -72,7 +72,6 @@ struct ExpandSmem {
     int32_t ul_in;                     // bottom-up list mode: buffer holding this pass's unvisited list, or -1
     int32_t ul_n;                      // entries of that list
     int32_t ul_base;                   // where this chunk's still-unvisited vertices go in the next list
-    int32_t solo_stop;                 // the solo phase writes its frontier out (CTA-uniform decision)
     int32_t run_count;                 // expand: runs of a sub-round that spans more than B entries
     uint32_t win_word[B];              // bottom-up windows: the window's visited words, discoveries OR'ed in
     unsigned long long scan_warp[B / 32];
@@ -567,14 +566,13 @@ template <int B, bool PRED, bool FUSED_CULL, bool LISTS = false>
 __device__ __forceinline__ void expand_range(const BfsParams &p, const VertexFrontier &in, ExpandSmem<B, PRED> &s,
                                              int level, int pass, const VertexFrontier &vout,
                                              const EdgeFrontier &eout, unsigned long long *qe_out,
-                                             unsigned &bar_phase, int part, int parts,
-                                             unsigned long long skip_above = ~0ull)
+                                             unsigned &bar_phase, unsigned long long skip_above = ~0ull)
 {
     const int tid = threadIdx.x;
     const int q = s.q, E = s.E;
     constexpr int PER = kChunkMax / B;  // sub-round positions per thread
     int rs, re;
-    cta_range(E, part, parts, rs, re);
+    cta_range(E, blockIdx.x, gridDim.x, rs, re);
     if (rs >= re) return;
     int i_cur = ld_cg(in.cf + rs / kChunkGrain);  // entry owning position rs
     if (FUSED_CULL) stamp(p, pass, 0);
@@ -2003,7 +2001,6 @@ __device__ __forceinline__ bool choose_bottom_up(const BfsParams &p, bool was_bo
 // Level drivers
 // ------------------------------------------------------------------------------------
 
-
 __device__ __forceinline__ unsigned long long ld_cg64(const unsigned long long *p)
 {
     unsigned long long v;
@@ -2708,8 +2705,7 @@ __global__ void __launch_bounds__(B, 1024 / B) ec_kernel(BfsParams p)
                                                &p.st->qe[(pass + 1) % 3], nullptr, skip_above);
             } else {
                 expand_range<B, PRED, true, LISTS>(p, p.vf[level & 1], s, level, pass, p.vf[(level + 1) & 1],
-                                                   p.ef[0], &p.st->qe[(pass + 1) % 3], bar_phase, blockIdx.x,
-                                                   gridDim.x, skip_above);
+                                                   p.ef[0], &p.st->qe[(pass + 1) % 3], bar_phase, skip_above);
             }
         }
         __syncthreads();
@@ -2784,7 +2780,7 @@ __global__ void __launch_bounds__(B, 1024 / B) edge_kernel(BfsParams p)
                         expand_range_warp<B, PRED, false>(p, p.vf[0], s, level, p.vf[1], nullptr, &p.ef[out_idx]);
                     else
                         expand_range<B, PRED, false>(p, p.vf[0], s, level, pass, p.vf[1], p.ef[out_idx], nullptr,
-                                                     bar_phase, blockIdx.x, gridDim.x);
+                                                     bar_phase);
                 }
                 __syncthreads();
                 completed_level = true;
