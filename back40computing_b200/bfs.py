@@ -262,19 +262,22 @@ class EnactorExpandContract(_Enactor):
 
 
 class EnactorContractExpand(_Enactor):
-    """enactor_contract_expand.cuh:61 -- edge frontiers, fused contract+expand."""
+    """enactor_contract_expand.cuh:61 -- edge frontiers (per-level launches; a fused
+    search keeps none)."""
     STRATEGY = CONTRACT_EXPAND
     FRONTIER = EDGE_FRONTIERS
 
 
 class EnactorTwoPhase(_Enactor):
-    """enactor_two_phase.cuh:68 -- separate contract and expand kernels per level."""
+    """enactor_two_phase.cuh:68 -- separate contract and expand kernels per level (a
+    fused search is one launch)."""
     STRATEGY = TWO_PHASE
     FRONTIER = MIXED_FRONTIERS
 
 
 class EnactorHybrid(_Enactor):
-    """enactor_hybrid.cuh:64 -- fused contract-expand, two-phase while saturated."""
+    """enactor_hybrid.cuh:64 -- one fused launch (the reference's two-phase launches of
+    saturated levels have no counterpart: a fused search keeps no edge frontier)."""
     STRATEGY = HYBRID
     FRONTIER = EDGE_FRONTIERS
 

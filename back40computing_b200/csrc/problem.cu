@@ -195,7 +195,7 @@ b40c_bfs_policy default_policy(int strategy)
     pol.chunk_edges = dev::kChunkMax;
     pol.warp_gather_threshold = 32;
     pol.cta_gather_threshold = 512;
-    pol.saturation_quit = 512;  // SATURATION_QUIT = 4 * 128 (enactor_hybrid.cuh:571)
+    pol.saturation_quit = 512;  // SATURATION_QUIT = 4 * 128 (enactor_hybrid.cuh:571); nothing reads it
     pol.warp_cull = 0;
     pol.bitmask_precheck = 1;
     pol.bottom_up_alpha = 14;  // Beamer et al.'s defaults

@@ -1,7 +1,8 @@
 /*
  * Contract-expand enactor (drop-in for b40c/graph/bfs/enactor_contract_expand.cuh:61-604):
  * edge frontiers; each level contracts the incoming edge frontier (visited
- * test-and-set, labelling) and expands the survivors into the next one.
+ * test-and-set, labelling) and expands the survivors into the next one.  A
+ * fused search does both in one pass and keeps no edge frontier.
  */
 #pragma once
 #include "enactor_base.cuh"

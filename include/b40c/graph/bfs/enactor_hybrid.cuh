@@ -1,7 +1,8 @@
 /*
- * Hybrid enactor (drop-in for b40c/graph/bfs/enactor_hybrid.cuh:64-758): the fused
- * contract-expand kernel while the edge frontier is small, two-phase level
- * launches while it exceeds gridDim x saturation_quit items.
+ * Hybrid enactor (drop-in for b40c/graph/bfs/enactor_hybrid.cuh:64-758): one fused
+ * launch for the whole search.  The reference leaves its fused kernel for two-phase
+ * launches while the edge frontier is saturated; a fused search here keeps no edge
+ * frontier to saturate.
  */
 #pragma once
 #include "enactor_base.cuh"

@@ -1,7 +1,7 @@
 /*
  * Two-phase enactor (drop-in for b40c/graph/bfs/enactor_two_phase.cuh:68-772): one
- * vertex and one edge frontier; separate contract and expand phases per
- * level (separate launches when iterative).
+ * vertex and one edge frontier; separate contract and expand launches per
+ * level when iterative, one launch without an edge frontier when fused.
  */
 #pragma once
 #include "enactor_base.cuh"

@@ -77,12 +77,19 @@ enum {
 
 /* Runtime kernel policy (replaces the reference's compile-time KernelPolicy
  * template parameters, e.g. enactor_contract_expand.cuh:339-373).  A zero
- * field means "use the tuned default". */
+ * field means "use the tuned default"; b40c_bfs_default_policy gives the values
+ * that stand behind the zeros, except threads and ctas_per_sm, where a zero also
+ * follows the search and the graph (below). */
 typedef struct b40c_bfs_policy {
-    int32_t threads;               /* CTA size: 128, 256 or 512 (default 256; b40c_bfs_enact with no policy
-                                      at all runs 512 for the distance searches of expand-contract,
-                                      contract-expand, two-phase and hybrid) */
-    int32_t ctas_per_sm;           /* resident CTAs per SM for persistent grids (0 = occupancy limit) */
+    int32_t threads;               /* CTA size: 128, 256 or 512.  0, or no policy: 512 for searches and
+                                      batches, but 256 where bottom_up_list, a subgrid_frontier_edges
+                                      above 0 or warp_contract -1 asks for it, and in a query server
+                                      whose batches share the SMs.  (b40c_bfs_default_policy says 256:
+                                      pass 0 instead to follow this rule) */
+    int32_t ctas_per_sm;           /* resident CTAs per SM.  0: one 512-thread CTA on small graphs
+                                      (direction-optimizing searches up to 2^19 vertices, others up to 2^21
+                                      edges, batches up to 2^16 vertices; per-level expand-contract
+                                      launches choose level by level), else as many as fit */
     int32_t chunk_edges;           /* edges (or edge-frontier items) per sub-round of a CTA's share of a level:
                                       a multiple of 32 in [256, 2048] (default 2048) */
     int32_t warp_gather_threshold; /* run length at or above which a warp gathers cooperatively (>= 32) */
@@ -92,8 +99,11 @@ typedef struct b40c_bfs_policy {
     int32_t warp_cull;             /* 1: drop duplicate neighbours within a warp before the bitmask test,
                                       -1: do not (default) */
     int32_t bitmask_precheck;      /* 1: read the visited word (through L1) before the atomic test-and-set
-                                      (default), 2: read it from L2 (never stale), -1: go straight to the
-                                      atomic (default of direction-optimizing) */
+                                      (default), 2: read it from L2 (never stale; levels kept in shared
+                                      memory by a team of CTAs read it through L1), -1: go straight to the
+                                      atomic (default of direction-optimizing).  CTA-wide passes of fewer
+                                      than 65,536 items and at most as many as vertices always go straight
+                                      to it, as do such team levels */
     int32_t queue_allocation;      /* frontier-slot allocation per tile of output: 1 = decoupled look-back
                                       over tile ids, 2 = one packed 64-bit atomicAdd; 0 = default */
     int32_t bottom_up_alpha;       /* direction-optimizing: go bottom-up when frontier edges exceed
@@ -185,7 +195,9 @@ const char *b40c_version(void);
 /* Number of CUDA devices visible (0 on a machine without a GPU). */
 int b40c_device_count(int *count);
 
-/* Fills *policy with the tuned default for a strategy. */
+/* Fills *policy with the default of every field for a strategy.  Passing it back
+ * fixes its threads (256) and leaves ctas_per_sm open; set threads to 0 for what a
+ * search without a policy runs. */
 int b40c_bfs_default_policy(int strategy, b40c_bfs_policy *policy);
 
 /* ---- problem (bfs::CsrProblem, csr_problem.cuh:72-756) ---------------------- */
